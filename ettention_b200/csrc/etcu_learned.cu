@@ -192,7 +192,33 @@ etcu_status make_map(etcu_warmstart* w, CUtensorMap* m, const Tensor& t, int bat
     return ETCU_OK;
 }
 
-constexpr size_t kSmemBudget = 200 * 1024;      // weight-gradient kernel
+// Tensor map of an NC8 tensor in rows of kTileX cells: the same bytes as 64-bit elements, two
+// to a cell, so that a whole row of 2 KB is the copy's inner dimension (with the 16-byte cells
+// of make_map as the inner dimension the copy engine handles one cell per clock).
+etcu_status make_row_map(etcu_warmstart* w, CUtensorMap* m, const Tensor& t, int batch, uint32_t by, uint32_t bz,
+                         uint32_t bc) {
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return wfail(w, ETCU_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
+    const cuuint64_t dims[4] = {(cuuint64_t)2 * t.g.X, (cuuint64_t)t.g.Y, (cuuint64_t)t.g.Z,
+                                (cuuint64_t)batch * (t.C / 8)};
+    const cuuint64_t strides[3] = {(cuuint64_t)16 * t.g.X, (cuuint64_t)16 * t.g.X * t.g.Y,
+                                   (cuuint64_t)16 * t.g.X * t.g.Y * t.g.Z};
+    const cuuint32_t box[4] = {2 * ws::kTileX, by, bz, bc};
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_INT64, 4, (void*)t.p, dims, strides, box, es,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return wfail(w, ETCU_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return ETCU_OK;
+}
+
+constexpr size_t kSmemBudget = 200 * 1024;      // weight-gradient kernel's stages
+// CTAs per tap group of the weight gradient, one resident CTA per multiprocessor in all.
+int wgrad_ranges(int sms, int cin, int cp) {
+    const int groups = cin <= 32 && cp <= 32 ? 1 : 3;  // ws::WgradShape<cin, cp>::kGroups
+    return (sms + groups - 1) / groups;
+}
+
 constexpr size_t kConvSmemMax = 232448 - 1024 - 512;  // persistent convolution: stages + resident weights
 constexpr size_t kResidentMax = 64 * 1024;       // weights kept in shared memory for the whole launch
 
@@ -359,29 +385,26 @@ ws::ConvDst dst(const Tensor& t, const Tensor* mask = nullptr) {
     return d;
 }
 
-template <int CIN>
+template <int CIN, int CP>
 etcu_status launch_wgrad_n(etcu_warmstart* w, const Tensor& in, const Tensor& dpre, int cout, int batch,
                            int* ranges_out) {
-    const int mode = CIN == 16 ? 0 : (CIN == 32 ? 1 : 2);
-    const int ny = mode == 2 ? 1 : 3, nz = mode == 0 ? 3 : 1;
-    const int ngroups = mode == 0 ? 1 : (mode == 1 ? 3 : 9);
+    using SH = ws::WgradShape<CIN, CP>;
     CUtensorMap mi, md;
-    etcu_status s = make_map(w, &mi, in, batch, ws::kHaloX, ny, nz, CIN / 8);
+    etcu_status s = make_row_map(w, &mi, in, batch, 3, SH::kNz, CIN / 8);
     if (s != ETCU_OK) return s;
-    s = make_map(w, &md, dpre, batch, ws::kTileX, 1, 1, dpre.C / 8);
+    s = make_row_map(w, &md, dpre, batch, 1, 1, CP / 8);
     if (s != ETCU_OK) return s;
     const Grid& g = in.g;
     const int ntiles = ((g.X + ws::kTileX - 1) / ws::kTileX) * g.Y * g.Z * batch;
-    int ranges = std::max(1, std::min(ntiles, (w->sms + ngroups - 1) / ngroups));
-    const uint32_t bbytes = (uint32_t)ws::kHaloX * ny * nz * 16u * (CIN / 8);
-    const uint32_t stage = (16u * ws::kTileX * 16u + bbytes + 1023u) & ~1023u;
-    int S = (int)std::max<size_t>(1, std::min<size_t>(4, kSmemBudget / stage));
-    const size_t smem = (size_t)S * stage + (2 * S + 1) * 8 + 16 + 1024;
+    const int ranges = std::max(1, std::min(ntiles, wgrad_ranges(w->sms, CIN, CP)));
+    const int S = (int)std::max<size_t>(1, std::min<size_t>(4, kSmemBudget / SH::kStage));
+    // at least 120 KB, so that one CTA (and its tensor memory) owns each SM
+    const size_t smem = std::max<size_t>((size_t)S * SH::kStage + (2 * S + 1) * 8 + 16 + 1024, 120 * 1024);
     const size_t need = (size_t)ranges * 27 * cout * CIN;
     if (need > w->partial_floats) return wfail(w, ETCU_ERR_STATE, "weight-gradient scratch too small");
     static std::atomic<unsigned long long> opted{0};
     if (w->device < 64 && !(opted.load() & (1ull << w->device))) {
-        WCK(w, cudaFuncSetAttribute(ws::wgrad_tc_kernel<CIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        WCK(w, cudaFuncSetAttribute(ws::wgrad_tc_kernel<CIN, CP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024));
         opted.fetch_or(1ull << w->device);
     }
@@ -391,14 +414,12 @@ etcu_status launch_wgrad_n(etcu_warmstart* w, const Tensor& in, const Tensor& dp
     a.Z = g.Z;
     a.batch = batch;
     a.in_c8 = in.C / 8;
-    a.out_c8 = dpre.C / 8;
     a.cout = cout;
-    a.group_mode = mode;
     a.ranges = ranges;
     a.partial = w->partial;
     a.stages = S;
     a.err = w->d_err;
-    ws::wgrad_tc_kernel<CIN><<<(unsigned)(ngroups * ranges), 128, smem, w->stream>>>(mi, md, a);
+    ws::wgrad_tc_kernel<CIN, CP><<<(unsigned)(SH::kGroups * ranges), 128, smem, w->stream>>>(mi, md, a);
     WCK(w, cudaGetLastError());
     *ranges_out = ranges;
     return ETCU_OK;
@@ -410,11 +431,16 @@ etcu_status wgrad(etcu_warmstart* w, int l, const Tensor& in, int cin_used, int 
     const LayerDef& d = kDefs[l];
     int ranges = 0;
     etcu_status s;
-    switch (in.C) {
-    case 16: s = launch_wgrad_n<16>(w, in, dpre, d.cout, batch, &ranges); break;
-    case 32: s = launch_wgrad_n<32>(w, in, dpre, d.cout, batch, &ranges); break;
-    case 64: s = launch_wgrad_n<64>(w, in, dpre, d.cout, batch, &ranges); break;
-    default: return wfail(w, ETCU_ERR_UNSUPPORTED, "no weight-gradient kernel for %d input channels", in.C);
+    switch (in.C * 100 + dpre.C) {
+    case 1616: s = launch_wgrad_n<16, 16>(w, in, dpre, d.cout, batch, &ranges); break;
+    case 1632: s = launch_wgrad_n<16, 32>(w, in, dpre, d.cout, batch, &ranges); break;
+    case 3216: s = launch_wgrad_n<32, 16>(w, in, dpre, d.cout, batch, &ranges); break;
+    case 3232: s = launch_wgrad_n<32, 32>(w, in, dpre, d.cout, batch, &ranges); break;
+    case 3264: s = launch_wgrad_n<32, 64>(w, in, dpre, d.cout, batch, &ranges); break;
+    case 6432: s = launch_wgrad_n<64, 32>(w, in, dpre, d.cout, batch, &ranges); break;
+    case 6464: s = launch_wgrad_n<64, 64>(w, in, dpre, d.cout, batch, &ranges); break;
+    default:
+        return wfail(w, ETCU_ERR_UNSUPPORTED, "no weight-gradient kernel for %d -> %d channels", in.C, dpre.C);
     }
     if (s != ETCU_OK) return s;
     const int n = 27 * d.cout * cin_used;
@@ -756,8 +782,7 @@ extern "C" etcu_status etcu_warmstart_create(etcu_context* ctx, const uint32_t r
         }
         for (int cin : {d.cin0, d.cin1}) {
             if (cin == 0) continue;
-            const int ngroups = cin == 16 ? 1 : (cin == 32 ? 3 : 9);
-            const size_t r = (size_t)(p->sms + ngroups - 1) / ngroups;
+            const size_t r = (size_t)wgrad_ranges(p->sms, cin, d.npad);
             max_partial = std::max(max_partial, r * 27 * d.cout * cin);
         }
     }

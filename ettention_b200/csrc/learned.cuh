@@ -84,6 +84,14 @@ __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, u
         "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
         : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2,
+                                            int c3) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(smem_u32(dst)),
+        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+        : "memory");
+}
 // 16-byte copy global -> shared; src_bytes 0 writes 16 zero bytes (no global read).
 __device__ __forceinline__ void cp_async16z(uint32_t dst, const void* src, uint32_t src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
@@ -811,51 +819,66 @@ __global__ void relayout_zfold_kernel(const float* __restrict__ W, int cout, int
 }
 
 // ---------------------------------------------------------------- weight gradient
-// dW[tap][co][ci] = sum over voxels v of dPre[v][co] * In[v + off(tap)][ci].  Per tile of
-// 128 voxels the K dimension of the MMA runs over voxels: A = dPre^T (M = co, padded to
-// 128 rows, MN-major: 8 channels contiguous per voxel row), B = the tap-shifted input
-// (N = ci, MN-major), D[co][ci] of every tap of the CTA's tap group accumulates in tensor
-// memory over all tiles the CTA takes.
+// dW[dz][dy][dx][co][ci] = sum over voxels v of dPre[v][co] * In[v + (dx, dy, dz) - 1][ci]
+// = sum over input voxels u of dPre[u - (dx - 1) along x][co] * In[u + (dy, dz) - 1][ci]:
+// a product with the voxels as K, in which every tap of a tap group is a row or a column.
+//   A (M, MN-major): the tile's 128 dPre cells loaded three times, moved by one cell along x
+//     each time; rows dx * CP + co (CP = channels of the dPre tensor, 16 / 32 / 64).
+//   B (N, MN-major): the 128-cell rows of In's halo as the tensor copy leaves them,
+//     [chunk][dz][dy]: consecutive groups of 8 columns lie 2 KB apart, so one descriptor
+//     spans all of them; columns ((chunk * NZ + dz) * 3 + dy) * 8 + channel.
+// So a 16-voxel K step of a 16-channel input is one MMA of 144 columns.  With one MMA per
+// tap (N = 16) the tensor cores read the 4 KB A operand from shared memory 27 times per K
+// step and one thread issued 216 MMAs per tile: 3.6 ms for a 16 -> 16 layer at 256 x 256 x
+// 128.  This form took 0.76 ms with 16-byte cells as the copies' inner dimension (one cell per
+// clock) and 0.24 ms with rows of 2 KB (tma_load_4d of a 64-bit view of the tensor; moving by
+// a cell is two elements, 16 bytes).  What bounds it is the operands' way from L2: 48 KB per
+// tile of 128 voxels (3.1 GB, 13 TB/s), against 0.54 GB (0.08 ms) from DRAM.
 struct WgradArgs {
     int X, Y, Z, batch;
     int in_c8;             // chunks per batch item of the input tensor
-    int out_c8;            // chunks per batch item of dPre (COUT / 8)
     int cout;              // real output channels (rows of D that are written)
-    int group_mode;        // 0: all 27 taps, box 130x3x3; 1: one dz (9 taps), box 130x3x1; 2: one (dz, dy), box 130x1x1
     int ranges;            // CTAs per tap group (voxel tiles are dealt round-robin)
     float* partial;        // [ranges][27][cout][CIN]
     int stages;
     unsigned* err;
 };
 
-template <int CIN>
+// All 27 taps in one CTA where the accumulators fit in tensor memory and two stages in
+// shared memory (up to 32 input channels and 32 output channels); else one dz (9 taps) per CTA.
+template <int CIN, int CP>
+struct WgradShape {
+    static constexpr int kGroups = CIN <= 32 && CP <= 32 ? 1 : 3;   // tap groups (CTA kinds)
+    static constexpr int kNz = kGroups == 1 ? 3 : 1;                // halo slices of a group
+    static constexpr int kRows = CIN / 8 * kNz * 3;                 // column groups of 8
+    static constexpr int kPlanes = 3 * (CP / 8);                    // row groups of 8
+    static constexpr int kMBlocks = (kPlanes + 15) / 16;            // MMAs of 128 rows
+    static constexpr int kNSplit = kRows * 8 > 256 ? 2 : 1;         // MMAs of at most 256 columns
+    static constexpr int kN = kRows * 8 / kNSplit;
+    static constexpr uint32_t kRow = kTileX * 16u;                  // one row of cells, one chunk
+    static constexpr uint32_t kA = kPlanes * kRow, kB = kRows * kRow;
+    static constexpr uint32_t kStage = (kA + kB + 1023u) & ~1023u;
+    static constexpr int kUsed = kMBlocks * kRows * 8;              // tensor-memory columns
+    static constexpr uint32_t kCols = kUsed <= 128 ? 128 : kUsed <= 256 ? 256 : 512;
+    static_assert(kUsed <= 512 && kN % 16 == 0, "accumulators must fit in tensor memory");
+    // rows past 3 * CP of the last 128 are never read back; their operand reads stay in the stage
+    static_assert(kMBlocks * 16 * kRow <= kA + kB, "A operand reads must stay inside the stage");
+};
+
+template <int CIN, int CP>
 __global__ void __launch_bounds__(128) wgrad_tc_kernel(const __grid_constant__ CUtensorMap in_map,
                                                        const __grid_constant__ CUtensorMap dpre_map, WgradArgs a) {
-    static_assert(CIN == 16 || CIN == 32 || CIN == 64, "input chunks of 16, 32 or 64 channels");
-    constexpr uint32_t kA = 16u * kTileX * 16u;  // dPre: 16 planes of 128 voxel rows (M = 128)
-    constexpr uint32_t kIdesc = idesc_bf16(128, CIN, 1, 1);
+    using SH = WgradShape<CIN, CP>;
+    constexpr uint32_t kIdesc = idesc_bf16(128, SH::kN, 1, 1);
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const int mode = a.group_mode;
-    const int ny = mode == 2 ? 1 : 3, nz = mode == 0 ? 3 : 1;
-    const int ntaps = mode == 0 ? 27 : (mode == 1 ? 9 : 3);
-    const uint32_t bplane = (uint32_t)kHaloX * ny * nz * 16u;
-    const uint32_t bbytes = bplane * (CIN / 8);
-    const uint32_t stage = (kA + bbytes + 1023u) & ~1023u;
     const int S = a.stages;
-    uint64_t* full = (uint64_t*)(smem + S * stage);
+    uint64_t* full = (uint64_t*)(smem + S * SH::kStage);
     uint64_t* empty = full + S;
     uint64_t* done = empty + S;
     uint32_t* tmem_slot = (uint32_t*)(done + 1);
-    const uint32_t cols_needed = (uint32_t)ntaps * CIN;
-    const uint32_t ncols = cols_needed <= 32 ? 32 : cols_needed <= 64 ? 64 : cols_needed <= 128 ? 128
-                           : cols_needed <= 256 ? 256 : 512;
-
-    const int ngroups = mode == 0 ? 1 : (mode == 1 ? 3 : 9);
-    const int g = blockIdx.x % ngroups;
-    const int r = blockIdx.x / ngroups;
-    const int gdz = mode == 2 ? g / 3 : g;  // dz of the group (modes 1, 2)
-    const int gdy = mode == 2 ? g % 3 : 0;  // dy of the group (mode 2)
+    const int g = blockIdx.x % SH::kGroups;  // dz of the group when there are three
+    const int r = blockIdx.x / SH::kGroups;
     const int ntx = (a.X + kTileX - 1) / kTileX;
     const int ntiles = ntx * a.Y * a.Z * a.batch;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -868,12 +891,11 @@ __global__ void __launch_bounds__(128) wgrad_tc_kernel(const __grid_constant__ C
         mbar_init(done, 1);
         mbar_fence_init();
     }
-    if (warp == 0) tmem_alloc(tmem_slot, ncols);
+    if (warp == 0) tmem_alloc(tmem_slot, SH::kCols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const uint32_t abytes = (uint32_t)a.out_c8 * kTileX * 16u;
 
     if (warp == 0 && lane == 0) {
         int i = 0;
@@ -884,18 +906,19 @@ __global__ void __launch_bounds__(128) wgrad_tc_kernel(const __grid_constant__ C
                 break;
             }
             int t = tile;
-            const int xt = t % ntx;
+            const int x0 = (t % ntx) * kTileX;
             t /= ntx;
             const int y = t % a.Y;
             t /= a.Y;
             const int z = t % a.Z;
             const int n = t / a.Z;
-            uint8_t* sa = smem + st * stage;
-            mbar_expect_tx(&full[st], abytes + bbytes);
-            tma_load_5d(sa, &dpre_map, &full[st], 0, xt * kTileX, y, z, n * a.out_c8);
-            const int by = mode == 2 ? y - 1 + gdy : y - 1;
-            const int bz = mode == 0 ? z - 1 : z - 1 + gdz;
-            tma_load_5d(sa + kA, &in_map, &full[st], 0, xt * kTileX - 1, by, bz, n * a.in_c8);
+            uint8_t* sa = smem + st * SH::kStage;
+            mbar_expect_tx(&full[st], SH::kA + SH::kB);
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx)
+                tma_load_4d(sa + dx * (CP / 8) * SH::kRow, &dpre_map, &full[st], 2 * (x0 + 1 - dx), y, z, n * (CP / 8));
+            tma_load_4d(sa + SH::kA, &in_map, &full[st], 2 * x0, y - 1, SH::kGroups == 1 ? z - 1 : z - 1 + g,
+                        n * a.in_c8);
         }
     } else if (warp == 1 && lane == 0) {
         int i = 0;
@@ -908,22 +931,18 @@ __global__ void __launch_bounds__(128) wgrad_tc_kernel(const __grid_constant__ C
                 break;
             }
             tc_fence_after();
-            const uint32_t abase = smem_u32(smem + st * stage);
-            const uint32_t bbase = abase + kA;
-#pragma unroll 1
-            for (int j = 0; j < ntaps; ++j) {
-                int dz, dy, dx;
-                if (mode == 0) { dz = j / 9; dy = (j / 3) % 3; dx = j % 3; }
-                else if (mode == 1) { dz = 0; dy = j / 3; dx = j % 3; }
-                else { dz = 0; dy = 0; dx = j; }
-                const uint32_t boff = (uint32_t)(((dz * ny + dy) * kHaloX + dx) * 16);
+            const uint32_t base = smem_u32(smem + st * SH::kStage);
+            const uint64_t ad = sdesc(base, 128, SH::kRow), bd = sdesc(base + SH::kA, 128, SH::kRow);
 #pragma unroll
-                for (int k = 0; k < kTileX / 16; ++k) {
-                    const uint64_t ad = sdesc(abase + k * 256u, 128, kTileX * 16u);
-                    const uint64_t bd = sdesc(bbase + boff + k * 256u, 128, bplane);
-                    umma_bf16(tmem + (uint32_t)(j * CIN), ad, bd, kIdesc, (i > 0 || k > 0) ? 1u : 0u);
-                }
-            }
+            for (int k = 0; k < kTileX / 16; ++k)
+#pragma unroll
+                for (int mb = 0; mb < SH::kMBlocks; ++mb)
+#pragma unroll
+                    for (int ns = 0; ns < SH::kNSplit; ++ns)
+                        umma_bf16(tmem + (uint32_t)((mb * SH::kNSplit + ns) * SH::kN),
+                                  ad + (uint64_t)((mb * 16 * SH::kRow + k * 256u) >> 4),
+                                  bd + (uint64_t)((ns * (SH::kRows / SH::kNSplit) * SH::kRow + k * 256u) >> 4), kIdesc,
+                                  (i > 0 || k > 0) ? 1u : 0u);
             umma_commit(&empty[st]);
         }
         if (ok) umma_commit(done);
@@ -933,23 +952,30 @@ __global__ void __launch_bounds__(128) wgrad_tc_kernel(const __grid_constant__ C
     if (!got && threadIdx.x == 0) atomicOr(a.err, kErrWaitDone);
     __syncwarp();
     tc_fence_after();
-    if (got && warp * 32 < a.cout) {
-        // lane = output channel co; columns j * CIN + ci
-        const int co = warp * 32 + lane;
-        const int tap_base = mode == 0 ? 0 : (mode == 1 ? gdz * 9 : gdz * 9 + gdy * 3);
-        for (int j = 0; j < ntaps; ++j) {
+    if (got) {
 #pragma unroll
-            for (int c = 0; c < CIN / 16; ++c) {
+        for (int mb = 0; mb < SH::kMBlocks; ++mb) {
+            const int row0 = mb * 128 + warp * 32;
+            if (row0 >= 3 * CP) continue;
+            const int m = row0 + lane;
+            const int dx = m / CP, co = m % CP;
+#pragma unroll 1
+            for (int rr = 0; rr < SH::kRows; rr += 2) {  // 16 columns: two halo rows
                 uint32_t v[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * CIN + c * 16), v);
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((mb * SH::kRows + rr) * 8), v);
                 tmem_wait_ld();
-                if (co < a.cout) {
-                    float* dst = a.partial + (((size_t)r * 27 + tap_base + j) * a.cout + co) * CIN + c * 16;
+                if (dx >= 3 || co >= a.cout) continue;
 #pragma unroll
-                    for (int q = 0; q < 16; q += 4)
-                        *reinterpret_cast<float4*>(dst + q) = make_float4(
-                            __uint_as_float(v[q]), __uint_as_float(v[q + 1]), __uint_as_float(v[q + 2]),
-                            __uint_as_float(v[q + 3]));
+                for (int h = 0; h < 2; ++h) {
+                    const int row = rr + h;
+                    const int dy = row % 3, dz = SH::kGroups == 1 ? (row / 3) % 3 : g, chunk = row / (3 * SH::kNz);
+                    float* dst =
+                        a.partial + (((size_t)r * 27 + (dz * 3 + dy) * 3 + dx) * a.cout + co) * CIN + chunk * 8;
+#pragma unroll
+                    for (int q = 0; q < 8; q += 4)
+                        *reinterpret_cast<float4*>(dst + q) =
+                            make_float4(__uint_as_float(v[h * 8 + q]), __uint_as_float(v[h * 8 + q + 1]),
+                                        __uint_as_float(v[h * 8 + q + 2]), __uint_as_float(v[h * 8 + q + 3]));
                 }
             }
         }
@@ -958,7 +984,7 @@ __global__ void __launch_bounds__(128) wgrad_tc_kernel(const __grid_constant__ C
     __syncthreads();
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, ncols);
+        tmem_dealloc(tmem, SH::kCols);
     }
 }
 

@@ -153,3 +153,22 @@ def test_zstreamed_convolution_equals_per_tap_kernel(ctx, monkeypatch, res, batc
         ob, _ = W.forward(p, v, 0.5, bf16=True)
         for mode in ("0", "1"):
             assert _rel(outs[mode] - v, ob - v) <= FWD_TOL
+
+
+@pytest.mark.parametrize("res,batch", [((4, 4, 4), 1), ((128, 4, 4), 3), ((132, 8, 4), 1), ((260, 12, 8), 2)])
+def test_weight_gradients_at_tile_edges(ctx, res, batch):
+    """The weight-gradient products over tiles of 128 cells of a row, every tap a row or a
+    column of one product: the smallest volume (one voxel at level 3), rows of exactly one
+    tile, of one tile and 4 voxels, and of two tiles and 4, so that the copies moved by one
+    cell along x cross the volume's and the tile's ends.  The tolerance is GRAD_TOL, as for
+    the gradients above (BF16 storage is emulated; only the order of FP32 sums differs)."""
+    import torch
+    from oracle import warmstart_oracle as W
+    from ettention_b200.learned import WarmStartNet
+    p = _params(13)
+    v, t = _volumes(res, batch, 14)
+    with WarmStartNet(ctx, res, max_batch=batch, params=p, scale=0.7) as net:
+        _, g = net.gradients(torch.as_tensor(v).cuda(), torch.as_tensor(t).cuda(), batch)
+    _, g16 = W.loss_and_grad(p, v, t, 0.7, bf16=True)
+    for i, (wo, bo) in enumerate(W.layer_offsets()):
+        assert _rel(g[wo:bo], g16[wo:bo]) <= GRAD_TOL, f"layer {i}"
