@@ -527,17 +527,111 @@ void launch_bp_col(const BpArgs& a0, const BpColPlan& p, cudaStream_t st) {
     }
 }
 
+struct BpBlockPlan {
+    int threads = 0;  // x voxels per block
+    int ntaps = 0, zper = 0;
+};
+
+// Whether the window-staged block kernel applies to `n` views (host copies hvc[vid], one
+// sample pattern of nsamples per vid, vids in order) of a sub-volume, and its shape.  It takes
+// views tilted about y with 1/256 sampling and no mask, any voxel type, any x.
+//  - threads: rows of 64, 128 or 256 voxels, the width that leaves the fewest idle lanes, counting
+//    the 40 or so window entries that a block stages beside its own width;
+//  - zper: all kZ register slices, or as few as 8 while the grid would not give every
+//    multiprocessor 768 threads (its residency): a 128 x 128 x 64 block step is latency-bound.
+bool plan_bp_block(const etcu_volume* vol, const SlabConst& g, const ViewConst* hvc, const float4* hsmp, int nsamples,
+                   const uint32_t* vids, int n, BpBlockPlan& p) {
+    etcu_context* ctx = vol->ctx;
+    if (!ctx->bp_column || vol->mask || g.rx <= 0 || g.ry <= 0 || g.rz <= 0) return false;
+    if (nsamples < 1 || nsamples > 255 || g.ry > 65535) return false;
+    const int kz = bp_block_z(nsamples > 1);
+    int best = 0;
+    for (int t : {256, 128, 64}) {
+        const int tiles = (g.rx + t - 1) / t, cost = tiles * (t + 40);
+        if (best == 0 || cost < best) {
+            best = cost;
+            p.threads = t;
+        }
+    }
+    const int xtiles = (g.rx + p.threads - 1) / p.threads;
+    p.zper = kz;
+    while (p.zper > 8 && (long long)xtiles * ((g.rz + p.zper - 1) / p.zper) * g.ry * p.threads <
+                             768ll * device_sms(ctx->device))
+        p.zper -= 8;
+    const int zchunks = (g.rz + p.zper - 1) / p.zper;  // even shares of the slices
+    p.zper = std::min(p.zper, ((g.rz + zchunks - 1) / zchunks + 7) / 8 * 8);
+    double span = 0.0;
+    for (int i = 0; i < n; ++i) {
+        const uint32_t vid = vids ? vids[i] : 0;
+        const ViewConst& c = hvc[vid];
+        if (!row_constant(c)) return false;
+        for (int k = 0; k < nsamples; ++k) {
+            const float4& s = hsmp[(size_t)vid * nsamples + k];
+            for (int q = 0; q < 8; ++q) {
+                const double x = (q & 1) ? g.rx - 1 : 0, y = (q & 2) ? g.ry - 1 : 0, z = (q & 4) ? g.rz - 1 : 0;
+                const double u = (double)c.mat[0] * ((double)g.bmin.x + (x + 0.5) * g.vs.x + s.x) +
+                                 (double)c.mat[4] * ((double)g.bmin.y + (y + 0.5) * g.vs.y + s.y) +
+                                 (double)c.mat[8] * ((double)g.bmin.z + (z + 0.5) * g.vs.z + s.z) + c.mat[12];
+                if (!(u > -16000.0 && u < 16000.0)) return false;  // |256 u| < 2^22 for the tap split
+            }
+        }
+        span = std::max(span, std::fabs((double)c.mat[0] * g.vs.x) * (std::min(p.threads, g.rx) - 1) +
+                                  std::fabs((double)c.mat[8] * g.vs.z) * (std::min(p.zper, g.rz) - 1));
+    }
+    // first column two below the least coordinate's; at the other end the tap itself, a weight
+    // rounded up to the next texel and two columns of margin
+    p.ntaps = (int)std::ceil(span) + 7;
+    return p.ntaps <= 1024;
+}
+
+template <int kT, bool kMulti>
+void launch_bp_block_s(const BpBlockArgs& b, dim3 grid, size_t smem, etcu_voxel_type t, int device, cudaStream_t st) {
+    static std::atomic<unsigned long long> opted{0};
+    if (device < 64 && !(opted.load(std::memory_order_acquire) & (1ull << device))) {
+        cudaFuncSetAttribute(bp_block_kernel<kT, kMulti, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(bp_block_kernel<kT, kMulti, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(bp_block_kernel<kT, kMulti, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(bp_block_kernel<kT, kMulti, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        opted.fetch_or(1ull << device, std::memory_order_acq_rel);
+    }
+    switch (t) {
+    case ETCU_VOXEL_FLOAT32: bp_block_kernel<kT, kMulti, 0><<<grid, kT, smem, st>>>(b); break;
+    case ETCU_VOXEL_HALF16: bp_block_kernel<kT, kMulti, 1><<<grid, kT, smem, st>>>(b); break;
+    case ETCU_VOXEL_F16_MASTER: bp_block_kernel<kT, kMulti, 2><<<grid, kT, smem, st>>>(b); break;
+    case ETCU_VOXEL_BF16_MASTER: bp_block_kernel<kT, kMulti, 3><<<grid, kT, smem, st>>>(b); break;
+    }
+}
+
+void launch_bp_block(const BpArgs& a, const BpBlockPlan& p, etcu_voxel_type t, int device, cudaStream_t st) {
+    BpBlockArgs b{a, p.ntaps, p.zper, (a.slab.rx + p.threads - 1) / p.threads};
+    const dim3 grid((unsigned)(b.xtiles * ((a.slab.rz + p.zper - 1) / p.zper)), (unsigned)a.slab.ry);
+    const size_t smem = bp_block_smem_bytes(a.nviews, a.nsamples, p.ntaps);
+    const bool multi = a.nsamples > 1;
+    if (p.threads == 256)
+        multi ? launch_bp_block_s<256, true>(b, grid, smem, t, device, st)
+              : launch_bp_block_s<256, false>(b, grid, smem, t, device, st);
+    else if (p.threads == 128)
+        multi ? launch_bp_block_s<128, true>(b, grid, smem, t, device, st)
+              : launch_bp_block_s<128, false>(b, grid, smem, t, device, st);
+    else
+        multi ? launch_bp_block_s<64, true>(b, grid, smem, t, device, st)
+              : launch_bp_block_s<64, false>(b, grid, smem, t, device, st);
+}
+
 // Back projection of a.nviews views; when their staged constants exceed the
 // shared-memory budget the views are split over consecutive launches, which
-// applies them in the same order.  `hvc` / `hsmp` are host copies of the single
-// view's constants and sample (they select the column-pipelined kernel).  Returns the
-// number of launches.
+// applies them in the same order.  `hvc` / `hsmp` are host copies of the views' constants
+// and sample patterns by view id (`vids`: the views' ids in order, NULL for the one view 0);
+// they select the column-pipelined kernel for one view and the window-staged one for several.
+// Returns the number of launches.
 uint32_t launch_bp(const etcu_volume* vol, const BpArgs& a0, bool persp, etcu_sampling sm, cudaStream_t st,
-                   bool row_const = false, const ViewConst* hvc = nullptr, const float4* hsmp = nullptr) {
+                   const ViewConst* hvc, const float4* hsmp, const uint32_t* vids) {
     const int dev = vol->ctx->device;
+    const uint32_t v0 = vids ? vids[0] : 0;
+    const bool row_const = row_constant(hvc[v0]);
     if (!persp && row_const && a0.nviews == 1 && a0.nsamples == 1 && sm != ETCU_SAMPLING_HW_TEXTURE) {
         BpColPlan plan;
-        if (sm == ETCU_SAMPLING_Q8 && hvc && hsmp && plan_bp_col(vol, a0.slab, *hvc, *hsmp, plan)) {
+        if (sm == ETCU_SAMPLING_Q8 && plan_bp_col(vol, a0.slab, hvc[v0], hsmp[v0], plan)) {
             launch_bp_col(a0, plan, st);
             return 1;
         }
@@ -545,8 +639,13 @@ uint32_t launch_bp(const etcu_volume* vol, const BpArgs& a0, bool persp, etcu_sa
         else launch_bp_sart_m<false>(a0, vol->type, sm, st);
         return 1;
     }
-    const size_t per_view = bp_smem_bytes(1, persp ? kBpZPersp : a0.nsamples);
-    const int max_views = (int)std::max<size_t>(1, (kBpSmemBudget - 16) / per_view);
+    BpBlockPlan block;
+    const bool staged = !persp && sm == ETCU_SAMPLING_Q8 &&
+                        plan_bp_block(vol, a0.slab, hvc, hsmp, a0.nsamples, vids, a0.nviews, block);
+    // the staged kernel's view constants stay within 32 KB, so that its blocks share an SM
+    const size_t per_view = staged ? (size_t)a0.nsamples * sizeof(BpBlockView)
+                                   : bp_smem_bytes(1, persp ? kBpZPersp : a0.nsamples);
+    const int max_views = (int)std::max<size_t>(1, ((staged ? 32 * 1024 : kBpSmemBudget) - 16) / per_view);
     uint32_t launches = 0;
     for (int c0 = 0; c0 < a0.nviews; c0 += max_views) {
         BpArgs a = a0;
@@ -555,7 +654,9 @@ uint32_t launch_bp(const etcu_volume* vol, const BpArgs& a0, bool persp, etcu_sa
         a.rl = a0.rl + (size_t)c0 * a0.rl_slot;
         if (a0.texs) a.texs = a0.texs + c0;
         const bool mask = a.mask != nullptr;
-        if (persp) {
+        if (staged) {
+            launch_bp_block(a, block, vol->type, dev, st);
+        } else if (persp) {
             if (mask) launch_bp_m<true, true>(a, vol->type, sm, dev, st);
             else launch_bp_m<true, false>(a, vol->type, sm, dev, st);
         } else {
@@ -1143,8 +1244,7 @@ etcu_status bp_one_slab(etcu_volume* vol, const etcu_view* view, const SlabConst
     a.use_max = vol->use_max;
     a.vmin = vol->vmin;
     a.vmax = vol->vmax;
-    launch_bp(vol, a, view->perspective != 0, sampling, ctx->stream, row_constant(a.inline_view), &a.inline_view,
-              &a.inline_samples[0]);
+    launch_bp(vol, a, view->perspective != 0, sampling, ctx->stream, &a.inline_view, &a.inline_samples[0], nullptr);
     CKL(ctx);
     return ETCU_OK;
 }
@@ -1362,10 +1462,8 @@ uint32_t issue_backward(etcu_recon* r, uint32_t first, uint32_t count, cudaStrea
         a.use_max = vol->use_max;
         a.vmin = vol->vmin;
         a.vmax = vol->vmax;
-        const uint32_t vid = r->order[first];
-        n += launch_bp(vol, a, r->persp, r->params.sampling, st, count == 1 && r->row_const[vid],
-                       &r->hvc[(size_t)s * r->n_input + vid],
-                       r->hsamples.empty() ? nullptr : &r->hsamples[(size_t)vid * r->nsamples]);
+        n += launch_bp(vol, a, r->persp, r->params.sampling, st, &r->hvc[(size_t)s * r->n_input],
+                       r->hsamples.data(), &r->order[first]);
     }
     return n;
 }

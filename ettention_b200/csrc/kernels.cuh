@@ -1238,6 +1238,194 @@ __global__ void __launch_bounds__(kBpColThreads, 4) bp_sart_column_kernel(const 
     cp_async_wait<0>();
 }
 
+// ---- block of views tilted about y: window-staged back projection (SIRT, blocks, WBP) ----
+// A block of kT threads owns kT consecutive x voxels of one volume row y over kZ slices, one
+// x per thread with its kZ voxels in registers, and applies the block's views to them in
+// order (the volume is read and written once per block of views, as in bp_parallel_kernel).
+// Per view (and sample) the two detector rows that row y projects to are blended once into
+// a shared-memory window of tap pairs over the columns that the brick projects to, the next
+// view's window while this one is applied; each voxel then takes one 16-byte shared load.
+// Coordinates, 1/256 weights and the update are those of bp_sart_column_kernel (two z voxels
+// per paired instruction), so results agree with bp_parallel_kernel's to a few ulps per update.
+// Lanes hold consecutive x: their taps lie cos(tilt) entries apart, free of bank conflicts
+// without padding.
+// bp_parallel_kernel spends about 84 thread instructions per voxel and view (four 8-byte
+// gathers, the blend of four taps, an IEEE-accurate quotient): 38.2 ms for the 61 views of a
+// 1024 x 1024 x 256 SIRT iteration, 4.93 ms at 512 x 512 x 128.  This one takes 11.9 and 1.56 ms
+// and is bound by issue (about 14 instructions) and the shared-memory pipe (16 bytes per voxel
+// and view, 7.3 ms at the former size) together.  With each thread forming the views' window
+// bounds and row weights itself instead of once per block it took 13.4 ms.
+// kMulti: nsamples > 1, averaged over the samples with a ray length (used counts in bytes).
+struct BpBlockArgs {
+    BpArgs a;
+    int ntaps;    // window entries, enough for every view's span over the brick
+    int zper;     // slices per block (a multiple of 8, at most kZ)
+    int xtiles;
+};
+
+// One view's (and sample's) constants for the block's brick, formed once.
+struct __align__(16) BpBlockView {
+    float mu0, mu2, mu3, cy1;  // column coordinate: (mu0 (cx + sx) + cy1) + mu2 (cz + sz) + mu3
+    float sx, sz, bw, lamd;    // second detector row's weight, lambda * chord
+    long long row;             // element offset of the first detector row in the (residual, length) slots
+    int x0lo, pad;             // first column of the window
+};
+
+__host__ __device__ constexpr int bp_block_z(bool multi) { return multi ? 16 : 32; }
+__host__ __device__ constexpr size_t bp_block_smem_bytes(int nviews, int nsamples, int ntaps) {
+    return (size_t)nviews * nsamples * sizeof(BpBlockView) + 2 * ((size_t)ntaps * 16 + 32 * 4);
+}
+
+template <int kT, bool kMulti, int kStore>
+__global__ void __launch_bounds__(kT, (kMulti ? 640 : 768) / kT) bp_block_kernel(const __grid_constant__ BpBlockArgs b) {
+    constexpr int kZ = bp_block_z(kMulti);
+    const BpArgs& a = b.a;
+    extern __shared__ __align__(16) unsigned char bp_smem[];
+    const int total = a.nviews * (kMulti ? a.nsamples : 1);
+    BpBlockView* sv = (BpBlockView*)bp_smem;
+    const uint32_t win0 = (uint32_t)total * (uint32_t)sizeof(BpBlockView);  // the two windows
+    const uint32_t win_bytes = (uint32_t)b.ntaps * 16u + 32u * 4u;
+    const SlabConst& g = a.slab;
+    const int tid = threadIdx.x;
+    const int xt = (int)blockIdx.x % b.xtiles, zc = (int)blockIdx.x / b.xtiles, y = blockIdx.y;
+    const int xa = xt * kT, xb = min(g.rx, xa + kT) - 1;
+    const int z0 = zc * b.zper, nzc = min(b.zper, g.rz - z0);
+    const bool on = xa + tid <= xb;
+    const int x = min(xa + tid, xb);  // threads past the row follow its last voxel
+    const float cx = fadd(g.bmin.x, fmul(fadd((float)x, 0.5f), g.vs.x));
+    const size_t plane = (size_t)g.rx * (size_t)g.ry;
+    const size_t base = (size_t)z0 * plane + (size_t)y * (size_t)g.rx + (size_t)x;
+
+    for (int i = tid; i < total; i += kT) {
+        const int p = kMulti ? i / a.nsamples : i, k = kMulti ? i - p * a.nsamples : 0;
+        const uint32_t vid = a.order ? a.order[a.first + p] : (a.first + p);
+        const ViewConst& vc = a.views ? a.views[vid] : a.inline_view;
+        const float4 s = a.samples ? a.samples[(size_t)vid * a.nsamples + k] : a.inline_samples[k];
+        const float cy = fadd(g.bmin.y, fmul(fadd((float)y, 0.5f), g.vs.y));
+        const float cxa = fadd(g.bmin.x, fmul(fadd((float)xa, 0.5f), g.vs.x));
+        const float cxb = fadd(g.bmin.x, fmul(fadd((float)xb, 0.5f), g.vs.x));
+        const float cza = fadd(g.bmin.z, fmul(fadd((float)z0, 0.5f), g.vs.z));
+        const float czb = fadd(g.bmin.z, fmul(fadd((float)(z0 + nzc - 1), 0.5f), g.vs.z));
+        BpBlockView v;
+        v.mu0 = vc.mat[0];
+        v.mu2 = vc.mat[8];
+        v.mu3 = vc.mat[12];
+        v.sx = s.x;
+        v.sz = s.z;
+        v.lamd = fmul(a.lambda, s.w);
+        const float py = fadd(cy, s.y);
+        v.cy1 = fmul(vc.mat[4], py);
+        // mat[1] is zero: every voxel of the row has the same detector row coordinate
+        int y0;
+        split_coord<kSampleQ8>(fadd(fadd(fmul(vc.mat[1], fadd(cxa, s.x)), fmul(vc.mat[5], py)), vc.mat[13]), a.H, y0,
+                               v.bw);
+        v.row = (long long)p * (long long)a.rl_slot + (long long)y0 * (long long)a.rl_pitch;
+        // the least column coordinate over the brick's corners (it is affine in x and z), with
+        // two columns of margin for the float rounding
+        const float lo = fminf(fmul(v.mu0, fadd(cxa, s.x)), fmul(v.mu0, fadd(cxb, s.x))) +
+                         fminf(fmul(v.mu2, fadd(cza, s.z)), fmul(v.mu2, fadd(czb, s.z))) + v.cy1 + v.mu3;
+        v.x0lo = (int)floorf(lo - 0.5f) - 2;
+        v.pad = 0;
+        sv[i] = v;
+    }
+    auto stage = [&](int i) {
+        const BpBlockView v = sv[i];
+        float4* taps = (float4*)(bp_smem + win0 + (uint32_t)(i & 1) * win_bytes);
+        float* K = (float*)(taps + b.ntaps);
+        if (tid < kZ) {  // slices past the brick repeat its last one, so their taps stay inside
+            const int z = z0 + min(tid, nzc - 1);
+            K[tid] = fmul(v.mu2, fadd(fadd(g.bmin.z, fmul(fadd((float)z, 0.5f), g.vs.z)), v.sz));
+        }
+        const float omb = fsub(1.f, v.bw);
+        const float2* r0 = a.rl + v.row;
+        const float2* r1 = r0 + a.rl_pitch;
+        const float2 zero = make_float2(0.f, 0.f);
+        for (int e = tid; e < b.ntaps; e += kT) {
+            const int x0 = v.x0lo + e;
+            const bool in0 = x0 >= -kPad && x0 < a.W + kPad, in1 = x0 + 1 >= -kPad && x0 + 1 < a.W + kPad;
+            const float2 p0 = in0 ? __ldg(r0 + x0) : zero, q0 = in1 ? __ldg(r0 + x0 + 1) : zero;
+            const float2 p1 = in0 ? __ldg(r1 + x0) : zero, q1 = in1 ? __ldg(r1 + x0 + 1) : zero;
+            const float2 P0 =
+                make_float2(fadd(fmul(omb, p0.x), fmul(v.bw, p1.x)), fadd(fmul(omb, p0.y), fmul(v.bw, p1.y)));
+            const float2 P1 =
+                make_float2(fadd(fmul(omb, q0.x), fmul(v.bw, q1.x)), fadd(fmul(omb, q0.y), fmul(v.bw, q1.y)));
+            taps[e] = make_float4(fmul(P0.x, v.lamd), P0.y, fmul(fsub(P1.x, P0.x), v.lamd), fsub(P1.y, P0.y));
+        }
+    };
+
+    float val[kZ];
+#pragma unroll
+    for (int j = 0; j < kZ; ++j) val[j] = j < nzc ? bp_load<kStore>(a, base + (size_t)j * plane) : 0.f;
+    float pv[kMulti ? kZ : 1];
+    uint32_t used[kMulti ? kZ / 4 : 1];
+    __syncthreads();  // the views' constants
+    stage(0);
+    __syncthreads();
+    int k = 0;  // sample of the view
+    for (int i = 0; i < total; ++i) {
+        if (i + 1 < total) stage(i + 1);
+        const BpBlockView v = sv[i];
+        const uint32_t win = win0 + (uint32_t)(i & 1) * win_bytes;
+        const float2* K2 = (const float2*)(bp_smem + win + (uint32_t)b.ntaps * 16u);
+        // byte offset of tap pair (bits >> 8) - 0x4B4000 - x0lo, the constant folded (mod 2^32)
+        const uint32_t tap0 = win - (uint32_t)(0x4B4000 + v.x0lo) * 16u;
+        const float2 au = splat(fadd(fmul(v.mu0, fadd(cx, v.sx)), v.cy1));
+        const float2 m12 = splat(v.mu3);
+        if (kMulti && k == 0) {
+#pragma unroll
+            for (int j = 0; j < kZ; ++j) pv[kMulti ? j : 0] = 0.f;
+#pragma unroll
+            for (int j = 0; j < kZ / 4; ++j) used[kMulti ? j : 0] = 0u;
+        }
+#pragma unroll
+        for (int j8 = 0; j8 < kZ; j8 += 8) {
+            if (j8 < nzc) {
+#pragma unroll
+                for (int j = j8; j < j8 + 8; j += 2) {
+                    const float2 u = add2(add2(au, K2[j / 2]), m12);
+                    const float2 f = __fadd2_rd(fma2(u, splat(256.f), splat(-127.5f)), splat(12582912.0f));
+                    const uint32_t b0 = __float_as_uint(f.x), b1 = __float_as_uint(f.y);
+                    const float2 w = q8_weight2(f2(q8_k1(b0), q8_k1(b1)));
+                    const float4 t0 = *(const float4*)(bp_smem + (uint32_t)(tap0 + ((b0 >> 4) & 0xFFFFFFF0u)));
+                    const float4 t1 = *(const float4*)(bp_smem + (uint32_t)(tap0 + ((b1 >> 4) & 0xFFFFFFF0u)));
+                    const float2 rl0 = fma2(splat(w.x), f2(t0.z, t0.w), f2(t0.x, t0.y));
+                    const float2 rl1 = fma2(splat(w.y), f2(t1.z, t1.w), f2(t1.x, t1.y));
+                    // ParallelBeamsBackProjection.cl:40-50: r * lambda * d / L where L > eps
+                    const float c0 = fmul(rl0.x, rcp_approx(rl0.y)), c1 = fmul(rl1.x, rcp_approx(rl1.y));
+                    const bool ok0 = rl0.y > kEps, ok1 = rl1.y > kEps;
+                    if (kMulti) {
+                        if (ok0) pv[j] = fadd(pv[j], c0);
+                        if (ok1) pv[j + 1] = fadd(pv[j + 1], c1);
+                        used[j / 4] += (ok0 ? 1u << (8 * (j % 4)) : 0u) + (ok1 ? 1u << (8 * (j % 4 + 1)) : 0u);
+                    } else {
+                        if (ok0) val[j] = fadd(val[j], c0);
+                        if (ok1) val[j + 1] = fadd(val[j + 1], c1);
+                    }
+                }
+            }
+        }
+        if (kMulti && ++k == a.nsamples) {
+            k = 0;
+#pragma unroll
+            for (int j = 0; j < kZ; ++j) {
+                const uint32_t n = (used[kMulti ? j / 4 : 0] >> (8 * (j % 4))) & 255u;
+                const float sum = pv[kMulti ? j : 0];
+                if (n != 0u) val[j] = fadd(val[j], n == 1u ? sum : div_fast(sum, (float)n));
+            }
+        }
+        if (kStore == 1 && (!kMulti || k == 0)) {
+#pragma unroll
+            for (int j = 0; j < kZ; ++j) val[j] = __half2float(__float2half_rn(val[j]));  // vstore_half per view
+        }
+        __syncthreads();  // window i is no longer read, window i + 1 is complete
+    }
+    if (on) {
+#pragma unroll
+        for (int j = 0; j < kZ; ++j)
+            if (j < nzc) bp_store<kStore>(a, base + (size_t)j * plane, val[j]);
+    }
+}
+
 // ---- fused SART step: back projection of one view, forward projection of the next ----
 // SART alternates BP(view p) and FP(view p + 1) (BlockIterativeReconstructionOperator.cpp:
 // 92-142 with blockSize 1).  For parallel views tilted about y both touch one xz plane
