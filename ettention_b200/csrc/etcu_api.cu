@@ -277,8 +277,8 @@ template <typename VoxT, bool kMask, int kPath>
 void launch_fp_t(const FpArgs& a, uint32_t nviews, cudaStream_t st) {
     dim3 block(128);
     dim3 grid;
-    if (kPath == kFpPathPerspective) grid = dim3((a.W + 15) / 16, (a.H + 7) / 8, nviews);
-    else grid = dim3((a.W + 127) / 128, a.H, nviews);
+    if (kPath == kFpPathPerspective) grid = dim3((a.W + 15) / 16 * nviews, (a.H + 7) / 8);
+    else grid = dim3((a.W + 127) / 128 * nviews, a.H);
     forward_project_kernel<VoxT, kMask, kPath><<<grid, block, 0, st>>>(a);
 }
 
