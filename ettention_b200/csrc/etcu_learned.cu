@@ -90,6 +90,11 @@ size_t layer_params(const LayerDef& d) { return (size_t)27 * d.cout * cin_total(
 // but the first, whose one input channel runs on the CUDA cores (the head's one output is
 // padded to 16).
 bool zfold_layer(int l) { return l > 0 && (kDefs[l].npad == 16 || kDefs[l].npad == 32); }
+// Layers whose whole input gradient (16 or 32 channels, one destination) has a z-streamed form.
+bool zfold_backward_layer(int l) {
+    const int n = cin_total(kDefs[l]);
+    return l > 0 && kDefs[l].cin1 == 0 && (n == 16 || n == 32);
+}
 
 size_t total_params() {
     size_t n = 0;
@@ -114,6 +119,7 @@ struct etcu_warmstart {
     __nv_bfloat16* wf[kLayers] = {};  // forward kernel layout
     __nv_bfloat16* wb[kLayers] = {};  // input-gradient kernel layout (input channels [0, dx_split))
     __nv_bfloat16* wb2[kLayers] = {}; // the rest of them, when the input gradient is split
+    __nv_bfloat16* wzb[kLayers] = {}; // input-gradient layout of the z-streamed kernel (or null)
     int adam_t = 0;
     // activations (level 1 / 2 / 3)
     Tensor x16, e1a, e1b, up1, d1a, d1b, dy16, gA1, gB1, gUp1, gSkip1;
@@ -377,6 +383,35 @@ etcu_status conv(etcu_warmstart* w, const ConvCall& c, int batch) {
     }
 }
 
+// The same on the z-streamed kernel, for 16 or 32 channels into one destination; `weights` in
+// its layout.
+etcu_status conv_zfold(etcu_warmstart* w, const ConvCall& c, const __nv_bfloat16* weights, int batch) {
+    const int rows = zfold_rows(c.n);
+    CUtensorMap m0, m1;
+    etcu_status s = make_map(w, &m0, *c.src0, batch, ws::kHaloX, rows + 2, 1, 2);
+    if (s != ETCU_OK) return s;
+    s = make_map(w, &m1, c.src1 ? *c.src1 : *c.src0, batch, ws::kHaloX, rows + 2, 1, 2);
+    if (s != ETCU_OK) return s;
+    ws::ZfoldArgs z{};
+    z.X = c.src0->g.X;
+    z.Y = c.src0->g.Y;
+    z.Z = c.src0->g.Z;
+    z.nsteps = c.nsteps0 + c.nsteps1;
+    z.nkp0 = c.nsteps0;
+    z.c8_0 = c.src0->C / 8;
+    z.c8_1 = c.src1 ? c.src1->C / 8 : 0;
+    z.w = weights;
+    z.bias = c.bias;
+    z.relu = c.relu ? 1 : 0;
+    z.dst = c.dst0;
+    z.head = c.head ? 1 : 0;
+    z.head_in = c.head_in;
+    z.head_out = c.head_out;
+    z.head_scale = c.head_scale;
+    z.err = w->d_err;
+    return c.n == 16 ? launch_zfold<16>(w, m0, m1, z, batch) : launch_zfold<32>(w, m0, m1, z, batch);
+}
+
 ws::ConvDst dst(const Tensor& t, const Tensor* mask = nullptr) {
     ws::ConvDst d;
     d.ptr = t.p;
@@ -452,9 +487,10 @@ etcu_status wgrad(etcu_warmstart* w, int l, const Tensor& in, int cin_used, int 
 
 etcu_status bias_grad(etcu_warmstart* w, int l, const Tensor& dpre, int batch) {
     const int c8 = dpre.C / 8;
-    dim3 grid((unsigned)std::max<size_t>(1, std::min<size_t>(256, (batch * dpre.g.plane() + 255) / 256)),
-              (unsigned)c8);
-    ws::channel_sum_kernel<<<grid, 256, 0, w->stream>>>(dpre.p, c8, batch, dpre.g.plane(), kDefs[l].cout,
+    // two blocks per multiprocessor and chunk; four 16-byte loads per thread at the least
+    dim3 grid((unsigned)std::max<size_t>(1, std::min<size_t>(2 * (size_t)w->sms, dpre.g.plane() / 1024)), (unsigned)c8,
+              (unsigned)batch);
+    ws::channel_sum_kernel<<<grid, 256, 0, w->stream>>>(dpre.p, c8, dpre.g.plane(), kDefs[l].cout,
                                                         w->grads + w->boff[l]);
     WCK(w, cudaGetLastError());
     return ETCU_OK;
@@ -477,6 +513,11 @@ etcu_status relayout(etcu_warmstart* w) {
         if (l > 0) {
             const int nsteps_b = (d.cout + 15) / 16;
             const int n0 = dx_split(d), n1 = cin_total(d) - n0;
+            if (w->wzb[l]) {
+                const int nz = nsteps_b * 9 * 2 * 3 * n0 * 8;
+                ws::relayout_zfold_backward_kernel<<<blocks(nz), 256, 0, w->stream>>>(
+                    w->params + w->woff[l], d.cout, cin_total(d), n0, nsteps_b, w->wzb[l]);
+            }
             const int nb0 = nsteps_b * 27 * 2 * n0 * 8;
             ws::relayout_backward_kernel<<<blocks(nb0), 256, 0, w->stream>>>(w->params + w->woff[l], d.cout,
                                                                              cin_total(d), 0, n0, nsteps_b, w->wb[l]);
@@ -517,26 +558,7 @@ etcu_status forward(etcu_warmstart* w, const float* d_in, float* d_out, int B, b
         c.relu = true;
         c.n = d.npad;
         c.dst0 = dst(out);
-        if (w->zfold && w->wz[l]) {  // 16 or 32 outputs: the z-streamed kernel
-            const int rows = zfold_rows(d.npad);
-            CUtensorMap m0, m1;
-            WTRY(make_map(w, &m0, s0, B, ws::kHaloX, rows + 2, 1, 2));
-            WTRY(make_map(w, &m1, s1 ? *s1 : s0, B, ws::kHaloX, rows + 2, 1, 2));
-            ws::ZfoldArgs z{};
-            z.X = s0.g.X;
-            z.Y = s0.g.Y;
-            z.Z = s0.g.Z;
-            z.nsteps = c.nsteps0 + c.nsteps1;
-            z.nkp0 = c.nsteps0;
-            z.c8_0 = s0.C / 8;
-            z.c8_1 = s1 ? s1->C / 8 : 0;
-            z.w = w->wz[l];
-            z.bias = c.bias;
-            z.relu = 1;
-            z.dst = c.dst0;
-            z.err = w->d_err;
-            return d.npad == 16 ? launch_zfold<16>(w, m0, m1, z, B) : launch_zfold<32>(w, m0, m1, z, B);
-        }
+        if (w->zfold && w->wz[l]) return conv_zfold(w, c, w->wz[l], B);  // 16 or 32 outputs
         return conv(w, c, B);
     };
     // first layer (one input channel) on the CUDA cores
@@ -565,23 +587,16 @@ etcu_status forward(etcu_warmstart* w, const float* d_in, float* d_out, int B, b
     // head (one output channel): out = v + scale * (conv(d1b) + b), as the z-streamed
     // tensor-core convolution (channel 0 of 16), or on the CUDA cores
     if (w->zfold && w->wz[10]) {
-        CUtensorMap m0;
-        WTRY(make_map(w, &m0, w->d1b, B, ws::kHaloX, zfold_rows(16) + 2, 1, 2));
-        ws::ZfoldArgs z{};
-        z.X = w->g1.X;
-        z.Y = w->g1.Y;
-        z.Z = w->g1.Z;
-        z.nsteps = 1;
-        z.nkp0 = 1;
-        z.c8_0 = w->d1b.C / 8;
-        z.w = w->wz[10];
-        z.bias = w->params + w->boff[10];
-        z.head = 1;
-        z.head_in = d_in;
-        z.head_out = d_out;
-        z.head_scale = w->scale;
-        z.err = w->d_err;
-        return launch_zfold<16>(w, m0, m0, z, B);
+        ConvCall c{};
+        c.src0 = &w->d1b;
+        c.nsteps0 = 1;
+        c.bias = w->params + w->boff[10];
+        c.n = 16;
+        c.head = true;
+        c.head_in = d_in;
+        c.head_out = d_out;
+        c.head_scale = w->scale;
+        return conv_zfold(w, c, w->wz[10], B);
     }
     ws::conv_head_kernel<<<end_grid, 256, 0, w->stream>>>(w->d1b.p, w->g1.X, w->g1.Y, w->g1.Z, B,
                                                           w->params + w->woff[10], w->params + w->boff[10], d_in,
@@ -595,8 +610,9 @@ etcu_status backward(etcu_warmstart* w, const float* d_in, const float* d_target
     WCK(w, cudaMemsetAsync(w->grads, 0, w->nparams * sizeof(float), w->stream));
     WCK(w, cudaMemsetAsync(w->d_loss, 0, sizeof(double), w->stream));
     const float grad_scale = 2.f / (float)((double)B * p1n);
-    ws::loss_grad_kernel<<<blocks((size_t)B * p1n), 256, 0, w->stream>>>(w->out, d_target, 1.f / w->scale,
-                                                                          grad_scale, p1n, B, w->dy16.p, w->d_loss);
+    const dim3 loss_grid((unsigned)std::min<size_t>(8 * (size_t)w->sms, (p1n + 255) / 256), (unsigned)B);
+    ws::loss_grad_kernel<<<loss_grid, 256, 0, w->stream>>>(w->out, d_target, 1.f / w->scale, grad_scale, p1n, w->dy16.p,
+                                                           w->d_loss);
     WCK(w, cudaGetLastError());
     // input gradient of layer l from dPre_l into `out` (two outputs for the two-source layers)
     auto dx = [&](int l, const Tensor& dpre, const Tensor& out0, const Tensor* mask0, const Tensor* out1) {
@@ -616,6 +632,9 @@ etcu_status backward(etcu_warmstart* w, const float* d_in, const float* d_target
             c.n0 = d.cin0;
             c.n = cin_total(d);
         }
+        // 16 or 32 channels: the z-streamed kernel, as in the forward pass (0.22 against 0.60 ms for a
+        // 16-channel gradient at 256 x 256 x 128); the 48 of layer 8 stay together (0.51 ms; 0.58 as two)
+        if (w->zfold && w->wzb[l]) return conv_zfold(w, c, w->wzb[l], B);
         etcu_status st = conv(w, c, B);
         if (st != ETCU_OK || !out1 || dx_split(d) == cin_total(d)) return st;
         ConvCall c2 = c;  // source 1's input gradient
@@ -778,6 +797,8 @@ extern "C" etcu_status etcu_warmstart_create(etcu_context* ctx, const uint32_t r
         if (l > 0) {
             const size_t per = (size_t)((d.cout + 15) / 16) * 27 * 2 * 8 * 2;
             WTRY(walloc(p, (void**)&p->wb[l], per * dx_split(d)));
+            if (zfold_backward_layer(l))
+                WTRY(walloc(p, (void**)&p->wzb[l], (size_t)((d.cout + 15) / 16) * 9 * 2 * 3 * cin_total(d) * 8 * 2));
             if (cin_total(d) > dx_split(d)) WTRY(walloc(p, (void**)&p->wb2[l], per * (cin_total(d) - dx_split(d))));
         }
         for (int cin : {d.cin0, d.cin1}) {

@@ -818,6 +818,31 @@ __global__ void relayout_zfold_kernel(const float* __restrict__ W, int cout, int
     out[i] = __float2bfloat16_rn(w);
 }
 
+// Input-gradient weights for conv_zfold_kernel: the output channels are the layer's nout input
+// channels, the input channels its cout outputs, W' = W[26 - tap] transposed:
+// [step][tap9][half][r = g * nout + ci][8] = W[26 - (g * 9 + tap9)][co][ci].
+__global__ void relayout_zfold_backward_kernel(const float* __restrict__ W, int cout, int cin_total, int nout,
+                                               int nsteps, __nv_bfloat16* __restrict__ out) {
+    const int nn = 3 * nout;
+    const int total = nsteps * 9 * 2 * nn * 8;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total) return;
+    int t = i;
+    const int j = t % 8;
+    t /= 8;
+    const int r = t % nn;
+    t /= nn;
+    const int half = t % 2;
+    t /= 2;
+    const int tap9 = t % 9;
+    const int step = t / 9;
+    const int g = r / nout, ci = r % nout;
+    const int co = step * 16 + half * 8 + j;
+    const float w =
+        (co < cout && ci < cin_total) ? W[((size_t)(26 - (g * 9 + tap9)) * cout + co) * cin_total + ci] : 0.f;
+    out[i] = __float2bfloat16_rn(w);
+}
+
 // ---------------------------------------------------------------- weight gradient
 // dW[dz][dy][dx][co][ci] = sum over voxels v of dPre[v][co] * In[v + (dx, dy, dz) - 1][ci]
 // = sum over input voxels u of dPre[u - (dx - 1) along x][co] * In[u + (dy, dz) - 1][ci]:
@@ -1004,25 +1029,45 @@ __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, int range
     grad[(size_t)tc * cin_total + ci_off + ci] = s;
 }
 
-// db[c] += sum over voxels of an NC8 tensor's channel c (batch items included).
-__global__ void channel_sum_kernel(const __nv_bfloat16* __restrict__ t, int c8, int batch, size_t plane,
-                                   int cout, float* __restrict__ db) {
-    // blockIdx.y = chunk; blockIdx.x strides the (batch, voxel) range
+// db[c] += sum over voxels of an NC8 tensor's channel c (batch items included).  Grid: (blocks
+// over the voxels, chunks, batch items).  HBM-bound: 16 bytes per thread and load, four loads
+// in flight; one set of atomics per block (with one per warp, the 32 K atomics on a layer's one or
+// two cache lines were the bound: all eleven layers of a 256 x 256 x 128 step 1.09 ms).
+__global__ void __launch_bounds__(256) channel_sum_kernel(const __nv_bfloat16* __restrict__ t, int c8, size_t plane,
+                                                          int cout, float* __restrict__ db) {
     const int chunk = blockIdx.y;
+    const uint4* src = reinterpret_cast<const uint4*>(t) + ((size_t)blockIdx.z * c8 + chunk) * plane;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const size_t total = (size_t)batch * plane;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t n = i / plane, v = i % plane;
+    auto add = [&](const uint4& q) {
         float f[8];
-        unpack_bf16x8(*reinterpret_cast<const uint4*>(t + ((n * c8 + chunk) * plane + v) * 8), f);
+        unpack_bf16x8(q, f);
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[j] += f[j];
+    };
+    const size_t step = (size_t)gridDim.x * 256;
+    size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    for (; i + 3 * step < plane; i += 4 * step) {
+        const uint4 q0 = __ldg(src + i), q1 = __ldg(src + i + step), q2 = __ldg(src + i + 2 * step),
+                    q3 = __ldg(src + i + 3 * step);
+        add(q0);
+        add(q1);
+        add(q2);
+        add(q3);
     }
+    for (; i < plane; i += step) add(__ldg(src + i));
+    __shared__ float part[8][8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         float s = acc[j];
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0 && chunk * 8 + j < cout) atomicAdd(&db[chunk * 8 + j], s);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][j] = s;
+    }
+    __syncthreads();
+    const int j = threadIdx.x;
+    if (j < 8 && chunk * 8 + j < cout) {
+        float s = 0.f;
+        for (int w = 0; w < 8; ++w) s += part[w][j];
+        atomicAdd(&db[chunk * 8 + j], s);
     }
 }
 
@@ -1283,23 +1328,30 @@ __global__ void upsample_backward_kernel(const __nv_bfloat16* __restrict__ fine,
 
 // Loss gradient of L = mean(((out - target) / scale)^2) with respect to the normalised
 // output y = out / scale, written as chunk 0 channel 0 of a 16-channel NC8 tensor (the
-// head convolution's padded output); sum of squares to `loss` (FP64, one atomic per warp).
-__global__ void loss_grad_kernel(const float* __restrict__ out, const float* __restrict__ target, float inv_scale,
-                                 float grad_scale, size_t plane, int batch, __nv_bfloat16* __restrict__ dy,
-                                 double* __restrict__ loss) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+// head convolution's padded output); sum of squares to `loss` (FP64).  Grid: (blocks over the
+// voxels, batch items).  HBM-bound (24 bytes per voxel); one atomic per block, since with one per warp the
+// atomics on the one address were the bound (0.43 ms at 256 x 256 x 128).
+__global__ void __launch_bounds__(256) loss_grad_kernel(const float* __restrict__ out, const float* __restrict__ target,
+                                                        float inv_scale, float grad_scale, size_t plane,
+                                                        __nv_bfloat16* __restrict__ dy, double* __restrict__ loss) {
+    const size_t n = blockIdx.y;
     double sq = 0.0;
-    if (i < (size_t)batch * plane) {
-        const float d = (out[i] - target[i]) * inv_scale;
-        sq = (double)d * d;
-        const size_t n = i / plane, p = i % plane;
+    for (size_t p = (size_t)blockIdx.x * 256 + threadIdx.x; p < plane; p += (size_t)gridDim.x * 256) {
+        const float d = (out[n * plane + p] - target[n * plane + p]) * inv_scale;
+        sq += (double)d * d;
         uint4 o;
         o.x = pack_bf16x2(grad_scale * d, 0.f);
         o.y = o.z = o.w = 0u;
         *reinterpret_cast<uint4*>(dy + ((n * 2) * plane + p) * 8) = o;
     }
+    __shared__ double part[8];
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if ((threadIdx.x & 31) == 0 && sq != 0.0) atomicAdd(loss, sq);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sq;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) sq += part[w];
+        atomicAdd(loss, sq);
+    }
 }
 
 // Adam on the FP32 master parameters.
