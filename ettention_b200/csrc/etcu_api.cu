@@ -1535,15 +1535,9 @@ void launch_fused_persistent(etcu_recon* r, cudaStream_t st) {
     q.error = r->d_fuse_ctl + g.ry + 1;
     q.window = r->fuse_window;
     q.withhold_row = r->ctx->fuse_withhold_row;
-    switch (vol->type) {
-    case ETCU_VOXEL_F16_MASTER:
-        sart_fused_persistent_kernel<1><<<r->fuse_grid, kFuseThreads, r->fuse_smem, st>>>(a, q);
-        break;
-    case ETCU_VOXEL_BF16_MASTER:
-        sart_fused_persistent_kernel<2><<<r->fuse_grid, kFuseThreads, r->fuse_smem, st>>>(a, q);
-        break;
-    default: sart_fused_persistent_kernel<0><<<r->fuse_grid, kFuseThreads, r->fuse_smem, st>>>(a, q); break;
-    }
+    a.zc = fuse_narrow_chunk(g.rx);
+    const int shadow = vol->type == ETCU_VOXEL_F16_MASTER ? 1 : (vol->type == ETCU_VOXEL_BF16_MASTER ? 2 : 0);
+    fused_persistent_kernel(shadow, fuse_narrow(g.rx))<<<r->fuse_grid, kFuseThreads, r->fuse_smem, st>>>(a, q);
 }
 
 uint32_t issue_fused_iteration(etcu_recon* r, cudaStream_t st) {
@@ -1564,13 +1558,22 @@ uint32_t issue_fused_iteration(etcu_recon* r, cudaStream_t st) {
     return n;
 }
 
-void fuse_limits(int dev, size_t smem, int& per_sm, int& persist_per_sm, int& sms) {
+void fuse_limits(int dev, size_t smem, size_t persist_smem, bool narrow, int& per_sm, int& persist_per_sm, int& sms) {
     static std::mutex mu;
     static std::vector<char> opted;
     // two attributes, not cudaGetDeviceProperties (milliseconds per call, once per reconstruction)
     int optin = 0, nsm = 0;
     const bool have_prop = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
                            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
+// The persistent kernel of a shadow kind, for narrow rows or wide ones.
+auto fused_persistent_kernel(int shadow, bool narrow) {
+    if (narrow)
+        return shadow == 1 ? sart_fused_persistent_kernel<1, true>
+                           : (shadow == 2 ? sart_fused_persistent_kernel<2, true> : sart_fused_persistent_kernel<0, true>);
+    return shadow == 1 ? sart_fused_persistent_kernel<1, false>
+                       : (shadow == 2 ? sart_fused_persistent_kernel<2, false> : sart_fused_persistent_kernel<0, false>);
+}
+
     if (!have_prop) cudaGetLastError();
     {
         std::lock_guard<std::mutex> lock(mu);
@@ -1581,12 +1584,9 @@ void fuse_limits(int dev, size_t smem, int& per_sm, int& persist_per_sm, int& sm
                 cudaFuncSetAttribute(sart_fused_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, full);
                 cudaFuncSetAttribute(sart_fused_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, full);
                 cudaFuncSetAttribute(sart_fused_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, full);
-                cudaFuncSetAttribute(sart_fused_persistent_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     persist);
-                cudaFuncSetAttribute(sart_fused_persistent_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     persist);
-                cudaFuncSetAttribute(sart_fused_persistent_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     persist);
+                for (int i = 0; i < 6; ++i)
+                    cudaFuncSetAttribute(fused_persistent_kernel(i % 3, i >= 3),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, persist);
             }
             cudaGetLastError();
             opted[dev] = 1;
@@ -1599,8 +1599,8 @@ void fuse_limits(int dev, size_t smem, int& per_sm, int& persist_per_sm, int& sm
         cudaGetLastError();
         per_sm = 0;
     }
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&persist_per_sm, sart_fused_persistent_kernel<0>, kFuseThreads,
-                                                      smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&persist_per_sm, fused_persistent_kernel(0, narrow), kFuseThreads,
+                                                      persist_smem) != cudaSuccess) {
         cudaGetLastError();
         persist_per_sm = 0;
     }
@@ -1708,7 +1708,7 @@ etcu_status plan_fused(etcu_recon* r, const std::vector<ViewConst>& vc, bool& ok
     const SlabConst& g = vol->slabs[0];
     if (g.rx % 2 != 0 || g.rx > 2 * kFuseThreads || g.rx + g.rz - 1 > kMaxDdaIterations) return ETCU_OK;
     std::vector<int> x0lo(N), ntaps(N);
-    size_t smem = 0;
+    size_t smem = 0, persist_smem = 0;
     for (uint32_t v = 0; v < N; ++v) {
         const ViewConst& c = vc[v];
         if (!c.fast2d || !row_constant(c) || c.hpitch.y != 0.f) return ETCU_OK;
@@ -1719,7 +1719,7 @@ etcu_status plan_fused(etcu_recon* r, const std::vector<ViewConst>& vc, bool& ok
         smem = std::max(smem, fuse_smem_bytes(g.rx, g.rz, plan.ntaps));
     }
     int per_sm = 0, persist_per_sm = 0, sms = 0;
-    fuse_limits(ctx->device, smem, per_sm, persist_per_sm, sms);
+    fuse_limits(ctx->device, smem, persist_smem, fuse_narrow(g.rx), per_sm, persist_per_sm, sms);
     if (per_sm < 1) return ETCU_OK;
     // detector rows of every (view, volume row)
     const size_t T = (size_t)N * (size_t)g.ry;
@@ -1730,7 +1730,7 @@ etcu_status plan_fused(etcu_recon* r, const std::vector<ViewConst>& vc, bool& ok
     if (!rows_ok) return ETCU_OK;
     if ((s = dalloc(ctx, (void**)&r->d_jrange, T * sizeof(int2))) != ETCU_OK) return s;
     CK(ctx, cudaMemcpyAsync(r->d_jrange, table.data(), T * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
-    r->fuse_smem = smem;
+    r->fuse_smem = persist_smem;
     ok = true;
     if (ctx->fused_persist && persist_per_sm >= 1 && sms > 0) {
         int window = 0;
@@ -1783,6 +1783,8 @@ etcu_status tune_fused_grid(etcu_recon* r) {
         choice = etcu_tune::search(ctx->stream, cands, [&](int b) {
             r->fuse_grid = (int)std::min<long long>((long long)b * r->fuse_sms, units);
             return issue_iteration(r, ctx->stream, nullptr) == ETCU_OK;
+        persist_smem = std::max(persist_smem, fuse_narrow(g.rx) ? fuse_narrow_smem_bytes(g.rx, g.rz, plan.ntaps)
+                                                                : fuse_smem_bytes(g.rx, g.rz, plan.ntaps));
         }, 2, &log);
         CK(ctx, cudaMemcpyAsync(vol->master, save, n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
         if (lowb) CK(ctx, cudaMemcpyAsync(vol->low, (char*)save + n * 4, lowb, cudaMemcpyDeviceToDevice, ctx->stream));

@@ -1491,10 +1491,25 @@ struct FuseArgs {
     float* part;                // non-null: view p + 1's (projection, ray length) of this sub-volume go to
                                 // part[pixel] and part[W * H + pixel] (kFpSeparateAccumulate into
                                 // zeros) instead of the residual (the z-slab block step)
+    int zc;                     // z rows per chunk of the narrow form (fuse_narrow_chunk)
 };
 
 __host__ __device__ constexpr size_t fuse_smem_bytes(int rx, int rz, int ntaps) {
     return (size_t)bp_col_tap_slots(ntaps) * 16 + ((size_t)rz * 4 + 15) / 16 * 16 + 2 * (size_t)kFuseZc * rx * 4;
+}
+
+// Narrow rows (kNarrow): with two voxels of a row per thread, a 128-voxel row would occupy 64 of the
+// 512 threads and a chunk's eight slices be updated one after the other, once per 1 KB of volume and
+// barrier.  Rows of at most half the block instead put 512 / (rx / 2, in whole warps) groups of
+// threads on different slices of a chunk, and a chunk holds as many slices as 16 KB do.
+// (128 x 128 x 64 over 61 views, five iterations: 5.60 -> 3.87 ms; a step there is a chain of
+// fetch, update and walk in one block per row, not work.)
+__host__ __device__ constexpr bool fuse_narrow(int rx) { return rx <= kFuseThreads; }
+__host__ __device__ constexpr int fuse_narrow_chunk(int rx) {
+    return 4096 / rx / 8 * 8 < kFuseZc ? kFuseZc : (4096 / rx / 8 * 8 > 64 ? 64 : 4096 / rx / 8 * 8);
+}
+__host__ __device__ constexpr size_t fuse_narrow_smem_bytes(int rx, int rz, int ntaps) {
+    return fuse_smem_bytes(rx, rz, ntaps) + 2 * (size_t)(fuse_narrow_chunk(rx) - kFuseZc) * rx * 4;
 }
 
 // Global loads of data that other blocks of the same launch write (the persistent
@@ -1532,7 +1547,7 @@ __device__ __forceinline__ float shadow_value(float v) {
 // the shadow stores it, so the forward projection sees what the separate forward
 // projector reads from the shadow; the master is updated in FP32 (the shadow itself is
 // refreshed by the last back projection of the iteration).
-template <bool kCoherent, int kKind = kUnitFused, int kThreads = kFuseThreads, int kShadow = 0>
+template <bool kCoherent, int kKind = kUnitFused, int kThreads = kFuseThreads, int kShadow = 0, bool kNarrow = false>
 __device__ __forceinline__ void fused_row_step(const FuseArgs& a, uint32_t p, int y, int x0lo, int ntaps,
                                                const float2* rl_in, float2* rl_out,
                                                unsigned char* fuse_smem) {
@@ -1542,7 +1557,11 @@ __device__ __forceinline__ void fused_row_step(const FuseArgs& a, uint32_t p, in
     float4* taps = (float4*)fuse_smem;
     float* K = (float*)(taps + bp_col_tap_slots(ntaps));
     float* buf = (float*)(fuse_smem + (size_t)bp_col_tap_slots(ntaps) * 16 + ((size_t)rz * 4 + 15) / 16 * 16);
-    const size_t chunk_elems = (size_t)kFuseZc * rx;
+    const int zc = kNarrow ? a.zc : kFuseZc;
+    const size_t chunk_elems = (size_t)zc * rx;
+    // the slice of a chunk that this thread starts at, and its stride (kNarrow: groups of gw threads)
+    const int gw = kNarrow ? (rx / 2 + 31) / 32 * 32 : kThreads;
+    const int zg = kNarrow ? tid / gw : 0, zgroups = kNarrow ? kThreads / gw : 1;
 
     // ---- back projection constants of view p (bp_sart_column_kernel, one item = row y)
     const uint32_t vb = kBP ? a.order[p] : a.order[p + 1];
@@ -1551,8 +1570,8 @@ __device__ __forceinline__ void fused_row_step(const FuseArgs& a, uint32_t p, in
     if (kBP)
         for (int z = tid; z < rz; z += kThreads)
             K[z] = fmul(vc.mat[8], fadd(fadd(g.bmin.z, fmul(fadd((float)z, 0.5f), g.vs.z)), s.z));
-    const int x2 = 2 * tid;
-    const bool on = x2 < rx;
+    const int x2 = 2 * (tid - zg * gw);
+    const bool on = x2 < rx && zg < zgroups;
     float A[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j)
@@ -1629,17 +1648,22 @@ __device__ __forceinline__ void fused_row_step(const FuseArgs& a, uint32_t p, in
         }
     }
     const bool up = sz >= 0;
-    const int nchunks = (rz + kFuseZc - 1) / kFuseZc;
+    const int nchunks = (rz + zc - 1) / zc;
     const size_t plane = (size_t)rx * (size_t)ry;
 
     // chunk c (in walk order) -> its first z row
-    auto chunk_z0 = [&](int c) { return (up ? c : nchunks - 1 - c) * kFuseZc; };
+    auto chunk_z0 = [&](int c) { return (up ? c : nchunks - 1 - c) * zc; };
     auto fetch = [&](int c) {
         if (c < nchunks && on) {
-            const int z0 = chunk_z0(c), z1 = min(rz, z0 + kFuseZc);
+            const int z0 = chunk_z0(c), z1 = min(rz, z0 + zc);
             float* dst = buf + (size_t)(c & 1) * chunk_elems + x2;
             const float* src = a.vol + ((size_t)z0 * ry + y) * rx + x2;
-            if (z1 - z0 == kFuseZc) {  // a whole chunk: its rows unrolled
+            if constexpr (kNarrow) {
+                const uint32_t d0 = smem_addr(dst);
+#pragma unroll 4
+                for (int z = z0 + zg; z < z1; z += zgroups)
+                    cp_async8(d0 + 4u * (uint32_t)((z - z0) * rx), src + (size_t)(z - z0) * plane);
+            } else if (z1 - z0 == kFuseZc) {  // a whole chunk: its rows unrolled
                 const uint32_t d0 = smem_addr(dst);
 #pragma unroll
                 for (int k = 0; k < kFuseZc; ++k) cp_async8(d0 + 4u * (uint32_t)(k * rx), src + (size_t)k * plane);
@@ -1652,16 +1676,16 @@ __device__ __forceinline__ void fused_row_step(const FuseArgs& a, uint32_t p, in
     // BP update of chunk c in place (this thread's two columns), written back to the volume
     auto update = [&](int c) {
         if (!kBP && kShadow && c < nchunks && on) {  // the walk reads the shadow's values
-            const int z0 = chunk_z0(c), z1 = min(rz, z0 + kFuseZc);
+            const int z0 = chunk_z0(c), z1 = min(rz, z0 + zc);
             float* cb = buf + (size_t)(c & 1) * chunk_elems;
-            for (int z = z0; z < z1; ++z) {
+            for (int z = z0 + zg; z < z1; z += zgroups) {
                 float2* slot = reinterpret_cast<float2*>(cb + (size_t)(z - z0) * rx + x2);
                 const float2 v = *slot;
                 *slot = make_float2(shadow_value<kShadow>(v.x), shadow_value<kShadow>(v.y));
             }
         }
         if (!kBP || c >= nchunks || !on) return;
-        const int z0 = chunk_z0(c), z1 = min(rz, z0 + kFuseZc);
+        const int z0 = chunk_z0(c), z1 = min(rz, z0 + zc);
         float* cb = buf + (size_t)(c & 1) * chunk_elems;
         float* dst = a.vol + ((size_t)z0 * ry + y) * rx + x2;
         auto voxel = [&](int z, float* d) {
@@ -1691,7 +1715,10 @@ __device__ __forceinline__ void fused_row_step(const FuseArgs& a, uint32_t p, in
             *reinterpret_cast<float2*>(d) = o;
             *slot = kShadow ? make_float2(shadow_value<kShadow>(o.x), shadow_value<kShadow>(o.y)) : o;
         };
-        if (z1 - z0 == kFuseZc) {  // a whole chunk: its rows unrolled
+        if constexpr (kNarrow) {
+#pragma unroll 4
+            for (int z = z0 + zg; z < z1; z += zgroups) voxel(z, dst + (size_t)(z - z0) * plane);
+        } else if (z1 - z0 == kFuseZc) {  // a whole chunk: its rows unrolled
 #pragma unroll
             for (int k = 0; k < kFuseZc; ++k) voxel(z0 + k, dst + (size_t)k * plane);
         } else {
@@ -1707,7 +1734,7 @@ __device__ __forceinline__ void fused_row_step(const FuseArgs& a, uint32_t p, in
     // -(rz - rx)); dt = min(rx, -nz).  Same values as dda_walk_xz's updates.
     const float nsdz = -sdz;
     auto walk = [&](int c) {
-        const int z0 = chunk_z0(c), z1 = min(rz, z0 + kFuseZc);
+        const int z0 = chunk_z0(c), z1 = min(rz, z0 + zc);
         const unsigned char* cb = (const unsigned char*)(buf + (size_t)(c & 1) * chunk_elems);
         const int dxo = 4 * sx, dzo = 4 * sz * rx;
 #pragma unroll
@@ -1846,7 +1873,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-template <int kShadow>
+template <int kShadow, bool kNarrow>
 __global__ void __launch_bounds__(kFuseThreads, 2)
     sart_fused_persistent_kernel(const __grid_constant__ FuseArgs a, const __grid_constant__ FusePersist q) {
     extern __shared__ __align__(16) unsigned char fuse_smem[];
@@ -1854,36 +1881,33 @@ __global__ void __launch_bounds__(kFuseThreads, 2)
     const uint32_t ry = (uint32_t)a.slab.ry;
     const uint32_t total = q.steps * ry;
     uint32_t* done = q.ctl + 1;
+    const int lane = (int)threadIdx.x;
     for (;;) {
-        if (threadIdx.x == 0) {
+        if (lane < 32) {  // warp 0 takes the unit; its lanes wait for one row each
             uint32_t u = total;
-            if (ld_acquire_u32(q.error) == 0) {
-                u = atomicAdd(q.ctl, 1u);
-                if (u < total) {
-                    const uint32_t p = u / ry;
-                    const int y = (int)(u - p * ry);
-                    if (p > 0) {
-                        const int lo = max(0, y - q.window), hi = min((int)ry - 1, y + q.window);
-                        const unsigned long long t0 = global_ns();
-                        for (int yy = lo; yy <= hi && u < total; ++yy)
-                            while (ld_acquire_u32(done + yy) < p) {
-                                if (global_ns() - t0 > kFuseWaitNs) {
-                                    atomicExch(q.error, 1u);
-                                    u = total;
-                                    break;
-                                }
-                                if (ld_acquire_u32(q.error) != 0) {  // another block gave up
-                                    u = total;
-                                    break;
-                                }
-                                __nanosleep(128);
-                            }
+            if (lane == 0 && ld_acquire_u32(q.error) == 0) u = atomicAdd(q.ctl, 1u);
+            u = __shfl_sync(0xffffffffu, u, 0);
+            if (u >= total) u = total;
+            const uint32_t p = u / ry;
+            if (u < total && p > 0) {
+                const int y = (int)(u - p * ry);
+                const int lo = max(0, y - q.window), hi = min((int)ry - 1, y + q.window);
+                const unsigned long long t0 = global_ns();
+                for (int base = lo; base <= hi && u < total; base += 32) {
+                    const uint32_t* row = done + min(base + lane, hi);
+                    while (!__all_sync(0xffffffffu, ld_acquire_u32(row) >= p)) {
+                        bool stop = global_ns() - t0 > kFuseWaitNs;
+                        if (stop) atomicExch(q.error, 1u);
+                        else stop = ld_acquire_u32(q.error) != 0;  // another block gave up
+                        if (__any_sync(0xffffffffu, stop)) {
+                            u = total;
+                            break;
+                        }
+                        __nanosleep(64);
                     }
-                } else {
-                    u = total;
                 }
             }
-            unit_s = u;
+            if (lane == 0) unit_s = u;
         }
         __syncthreads();
         const uint32_t u = unit_s;
@@ -1891,7 +1915,8 @@ __global__ void __launch_bounds__(kFuseThreads, 2)
         const uint32_t p = u / ry;
         const int y = (int)(u - p * ry);
         const int2 tw = q.tapwin[a.order[p]];
-        fused_row_step<true, kUnitFused, kFuseThreads, kShadow>(a, p, y, tw.x, tw.y, q.rl0 + (size_t)(p & 1) * q.rl_slot,
+        fused_row_step<true, kUnitFused, kFuseThreads, kShadow, kNarrow>(a, p, y, tw.x, tw.y,
+                                                                q.rl0 + (size_t)(p & 1) * q.rl_slot,
                                                                 q.rl0 + (size_t)((p + 1) & 1) * q.rl_slot, fuse_smem);
         __syncthreads();  // the unit's stores are issued and its shared memory is free
         if (threadIdx.x == 0 && !(p == 0 && y == q.withhold_row)) {
