@@ -2321,8 +2321,9 @@ struct WbpFilter {
     }
     etcu_status init(etcu_context* c, uint32_t fres) {
         ctx = c;
-        // rows of up to 16384 padded pixels: 64 KB of shared memory
-        CK(ctx, cudaFuncSetAttribute(wbp_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 16384 * 4));
+        // rows of up to 16384 padded pixels, and as many filter positions of which every other is a tap
+        CK(ctx, cudaFuncSetAttribute(wbp_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)wbp_smem_bytes(16384, 16384 / 2 + 2)));
         std::vector<float> t;
         std::vector<int> p;
         ramlak_taps(fres, t, p);
@@ -2334,13 +2335,14 @@ struct WbpFilter {
         CK(ctx, cudaMemcpyAsync(pos, p.data(), p.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
         return ETCU_OK;
     }
-    void launch(WbpArgs a, uint32_t fres, cudaStream_t st) const {
+    // n views of a.proj
+    void launch(WbpArgs a, uint32_t n, uint32_t fres, cudaStream_t st) const {
         a.Wu = (int)next_pow2(std::max<uint32_t>((uint32_t)a.W, fres));
         a.Hu = (int)next_pow2((uint32_t)a.H);
         a.ntaps = ntaps;
         a.taps = taps;
         a.tap_pos = pos;
-        wbp_filter_kernel<<<a.H, 256, (size_t)a.Wu * sizeof(float), st>>>(a);
+        wbp_filter_kernel<<<(unsigned)a.H * n, 128, wbp_smem_bytes(a.Wu, ntaps), st>>>(a);
     }
 };
 
@@ -2365,7 +2367,7 @@ extern "C" etcu_status etcu_wbp_filter(etcu_context* ctx, const float* d_in, flo
     a.out_f = d_out;
     a.W = (int)width;
     a.H = (int)height;
-    f.launch(a, filter_width, ctx->stream);
+    f.launch(a, 1, filter_width, ctx->stream);
     CKL(ctx);
     CK(ctx, cudaStreamSynchronize(ctx->stream));
     return ETCU_OK;
@@ -2408,17 +2410,16 @@ extern "C" etcu_status etcu_wbp(etcu_volume* vol, const etcu_view* views, uint32
         return s;
     }
     const SlabConst& full = vol->slabs[0];
-    for (uint32_t v = 0; v < n_views; ++v) {
-        WbpArgs a{};
-        a.proj = r->d_proj + (size_t)v * r->W * r->H;
-        a.out = r->rl + (size_t)v * r->rl_slot;
-        a.pitch = r->rl_pitch;
-        a.W = (int)r->W;
-        a.H = (int)r->H;
-        a.vc = r->hvc[v];
-        a.g = full;  // cmin / cmax: the complete box
-        f.launch(a, fres, ctx->stream);
-    }
+    WbpArgs a{};
+    a.proj = r->d_proj;
+    a.out = r->rl;
+    a.pitch = r->rl_pitch;
+    a.slot = r->rl_slot;
+    a.W = (int)r->W;
+    a.H = (int)r->H;
+    a.views = r->d_views;
+    a.g = full;  // cmin / cmax: the complete box
+    f.launch(a, n_views, fres, ctx->stream);
     issue_backward(r, 0, n_views, ctx->stream);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
