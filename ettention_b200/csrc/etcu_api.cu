@@ -689,6 +689,15 @@ void fill_fp_volume_ptrs(const etcu_volume* vol, const SlabConst& s, FpArgs& a) 
 
 etcu_status make_pair_texture(etcu_context* ctx, float2* base, size_t pitch_elems, uint32_t W, uint32_t H,
                               cudaTextureObject_t* out) {
+        // rows that the column kernel does not take (x no multiple of 4, 16-bit volumes), from
+        // the size at which they fill the chip with 32 slices per thread (501 x 363 x 179: 129 -> 92 us;
+        // smaller volumes leave the window's set-up exposed)
+        BpBlockPlan one;
+        if (sm == ETCU_SAMPLING_Q8 &&
+            (long long)a0.slab.rx * a0.slab.ry * a0.slab.rz >= 32ll * 768 * device_sms(dev) && plan_bp_block(vol, a0.slab, hvc, hsmp, 1, vids, 1, one)) {
+            launch_bp_block(a0, one, vol->type, dev, st);
+            return 1;
+        }
     cudaResourceDesc rd{};
     rd.resType = cudaResourceTypePitch2D;
     rd.res.pitch2D.devPtr = base;
