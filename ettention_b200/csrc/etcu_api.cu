@@ -618,6 +618,60 @@ void launch_bp_block(const BpArgs& a, const BpBlockPlan& p, etcu_voxel_type t, i
               : launch_bp_block_s<64, false>(b, grid, smem, t, device, st);
 }
 
+// Whether bp_persp_row_kernel applies to `n` perspective views of a sub-volume: 1/256 sampling,
+// one sample per voxel, no mask, no detector column or depth that depends on y, and a source
+// outside the sub-volume along some axis.  It forms about half the instructions per voxel of
+// bp_perspective_kernel, whose chunks run along z, so it is the faster one unless its last
+// 16-voxel chunk in y leaves more than a third of the work idle.
+bool plan_bp_persp_rows(const etcu_volume* vol, const BpArgs& a, etcu_sampling sm, const ViewConst* hvc,
+                        const uint32_t* vids) {
+    const SlabConst& g = a.slab;
+    if (!vol->ctx->bp_column || sm != ETCU_SAMPLING_Q8 || a.mask || a.persp_n != 1) return false;
+    const int chunks = (g.ry + kBpYPersp - 1) / kBpYPersp;
+    if (chunks > 65535 || (g.rx + 31) / 32 > 65535 || 3ll * chunks * kBpYPersp > 4ll * g.ry)
+        return false;
+    if (!(g.vs.x >= 1e-6f && g.vs.y >= 1e-6f && g.vs.z >= 1e-6f)) return false;
+    for (int i = 0; i < a.nviews; ++i) {
+        const ViewConst& c = hvc[vids ? vids[i] : 0];
+        if (!(c.mat[4] == 0.f && c.mat[7] == 0.f)) return false;
+        const float4 &s = c.source, &lo = g.bmin, &hi = g.bmax;
+        if (!(s.x < lo.x || s.x > hi.x || s.y < lo.y || s.y > hi.y || s.z < lo.z || s.z > hi.z)) return false;
+    }
+    return true;
+}
+
+template <int kStore, bool kClamp>
+void launch_bp_persp_rows_t(const BpArgs& a, int device, cudaStream_t st) {
+    static std::atomic<unsigned long long> opted{0};
+    if (device < 64 && !(opted.load(std::memory_order_acquire) & (1ull << device))) {
+        cudaFuncSetAttribute(bp_persp_row_kernel<kStore, kClamp>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kBpSmemBudget);
+        opted.fetch_or(1ull << device, std::memory_order_acq_rel);
+    }
+    const SlabConst& g = a.slab;
+    const dim3 grid((unsigned)((g.rz + 3) / 4), (unsigned)((g.rx + 8 * kBpRowWarps - 1) / (8 * kBpRowWarps)),
+                    (unsigned)((g.ry + kBpYPersp - 1) / kBpYPersp));
+    bp_persp_row_kernel<kStore, kClamp><<<grid, dim3(32, kBpRowWarps), bp_persp_row_smem_bytes(a.nviews), st>>>(a);
+}
+
+void launch_bp_persp_rows(const BpArgs& a, etcu_voxel_type t, int device, cudaStream_t st) {
+    const bool clamp = a.use_min || a.use_max;
+    switch (t) {
+    case ETCU_VOXEL_FLOAT32:
+        clamp ? launch_bp_persp_rows_t<0, true>(a, device, st) : launch_bp_persp_rows_t<0, false>(a, device, st);
+        break;
+    case ETCU_VOXEL_HALF16:
+        clamp ? launch_bp_persp_rows_t<1, true>(a, device, st) : launch_bp_persp_rows_t<1, false>(a, device, st);
+        break;
+    case ETCU_VOXEL_F16_MASTER:
+        clamp ? launch_bp_persp_rows_t<2, true>(a, device, st) : launch_bp_persp_rows_t<2, false>(a, device, st);
+        break;
+    case ETCU_VOXEL_BF16_MASTER:
+        clamp ? launch_bp_persp_rows_t<3, true>(a, device, st) : launch_bp_persp_rows_t<3, false>(a, device, st);
+        break;
+    }
+}
+
 // Back projection of a.nviews views; when their staged constants exceed the
 // shared-memory budget the views are split over consecutive launches, which
 // applies them in the same order.  `hvc` / `hsmp` are host copies of the views' constants
@@ -635,6 +689,15 @@ uint32_t launch_bp(const etcu_volume* vol, const BpArgs& a0, bool persp, etcu_sa
             launch_bp_col(a0, plan, st);
             return 1;
         }
+        // rows that the column kernel does not take (x no multiple of 4, 16-bit volumes), from
+        // the size at which they fill the chip with 32 slices per thread (501 x 363 x 179: 129 -> 92 us;
+        // smaller volumes leave the window's set-up exposed)
+        BpBlockPlan one;
+        if (sm == ETCU_SAMPLING_Q8 &&
+            (long long)a0.slab.rx * a0.slab.ry * a0.slab.rz >= 32ll * 768 * device_sms(dev) && plan_bp_block(vol, a0.slab, hvc, hsmp, 1, vids, 1, one)) {
+            launch_bp_block(a0, one, vol->type, dev, st);
+            return 1;
+        }
         if (a0.mask) launch_bp_sart_m<true>(a0, vol->type, sm, st);
         else launch_bp_sart_m<false>(a0, vol->type, sm, st);
         return 1;
@@ -642,6 +705,7 @@ uint32_t launch_bp(const etcu_volume* vol, const BpArgs& a0, bool persp, etcu_sa
     BpBlockPlan block;
     const bool staged = !persp && sm == ETCU_SAMPLING_Q8 &&
                         plan_bp_block(vol, a0.slab, hvc, hsmp, a0.nsamples, vids, a0.nviews, block);
+    const bool persp_rows = persp && plan_bp_persp_rows(vol, a0, sm, hvc, vids);
     // the staged kernel's view constants stay within 32 KB, so that its blocks share an SM
     const size_t per_view = staged ? (size_t)a0.nsamples * sizeof(BpBlockView)
                                    : bp_smem_bytes(1, persp ? kBpZPersp : a0.nsamples);
@@ -656,6 +720,8 @@ uint32_t launch_bp(const etcu_volume* vol, const BpArgs& a0, bool persp, etcu_sa
         const bool mask = a.mask != nullptr;
         if (staged) {
             launch_bp_block(a, block, vol->type, dev, st);
+        } else if (persp_rows) {
+            launch_bp_persp_rows(a, vol->type, dev, st);
         } else if (persp) {
             if (mask) launch_bp_m<true, true>(a, vol->type, sm, dev, st);
             else launch_bp_m<true, false>(a, vol->type, sm, dev, st);
@@ -689,15 +755,6 @@ void fill_fp_volume_ptrs(const etcu_volume* vol, const SlabConst& s, FpArgs& a) 
 
 etcu_status make_pair_texture(etcu_context* ctx, float2* base, size_t pitch_elems, uint32_t W, uint32_t H,
                               cudaTextureObject_t* out) {
-        // rows that the column kernel does not take (x no multiple of 4, 16-bit volumes), from
-        // the size at which they fill the chip with 32 slices per thread (501 x 363 x 179: 129 -> 92 us;
-        // smaller volumes leave the window's set-up exposed)
-        BpBlockPlan one;
-        if (sm == ETCU_SAMPLING_Q8 &&
-            (long long)a0.slab.rx * a0.slab.ry * a0.slab.rz >= 32ll * 768 * device_sms(dev) && plan_bp_block(vol, a0.slab, hvc, hsmp, 1, vids, 1, one)) {
-            launch_bp_block(a0, one, vol->type, dev, st);
-            return 1;
-        }
     cudaResourceDesc rd{};
     rd.resType = cudaResourceTypePitch2D;
     rd.res.pitch2D.devPtr = base;
@@ -1514,6 +1571,15 @@ void launch_fused_step(etcu_recon* r, uint32_t p, cudaStream_t st, const float2*
     }
 }
 
+// The persistent kernel of a shadow kind, for narrow rows or wide ones.
+auto fused_persistent_kernel(int shadow, bool narrow) {
+    if (narrow)
+        return shadow == 1 ? sart_fused_persistent_kernel<1, true>
+                           : (shadow == 2 ? sart_fused_persistent_kernel<2, true> : sart_fused_persistent_kernel<0, true>);
+    return shadow == 1 ? sart_fused_persistent_kernel<1, false>
+                       : (shadow == 2 ? sart_fused_persistent_kernel<2, false> : sart_fused_persistent_kernel<0, false>);
+}
+
 // All M - 1 fused steps in one launch; the row counters are cleared first.
 void launch_fused_persistent(etcu_recon* r, cudaStream_t st) {
     etcu_volume* vol = r->vol;
@@ -1574,15 +1640,6 @@ void fuse_limits(int dev, size_t smem, size_t persist_smem, bool narrow, int& pe
     int optin = 0, nsm = 0;
     const bool have_prop = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
                            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
-// The persistent kernel of a shadow kind, for narrow rows or wide ones.
-auto fused_persistent_kernel(int shadow, bool narrow) {
-    if (narrow)
-        return shadow == 1 ? sart_fused_persistent_kernel<1, true>
-                           : (shadow == 2 ? sart_fused_persistent_kernel<2, true> : sart_fused_persistent_kernel<0, true>);
-    return shadow == 1 ? sart_fused_persistent_kernel<1, false>
-                       : (shadow == 2 ? sart_fused_persistent_kernel<2, false> : sart_fused_persistent_kernel<0, false>);
-}
-
     if (!have_prop) cudaGetLastError();
     {
         std::lock_guard<std::mutex> lock(mu);
@@ -1726,6 +1783,8 @@ etcu_status plan_fused(etcu_recon* r, const std::vector<ViewConst>& vc, bool& ok
         x0lo[v] = plan.x0lo;
         ntaps[v] = plan.ntaps;
         smem = std::max(smem, fuse_smem_bytes(g.rx, g.rz, plan.ntaps));
+        persist_smem = std::max(persist_smem, fuse_narrow(g.rx) ? fuse_narrow_smem_bytes(g.rx, g.rz, plan.ntaps)
+                                                                : fuse_smem_bytes(g.rx, g.rz, plan.ntaps));
     }
     int per_sm = 0, persist_per_sm = 0, sms = 0;
     fuse_limits(ctx->device, smem, persist_smem, fuse_narrow(g.rx), per_sm, persist_per_sm, sms);
@@ -1792,8 +1851,6 @@ etcu_status tune_fused_grid(etcu_recon* r) {
         choice = etcu_tune::search(ctx->stream, cands, [&](int b) {
             r->fuse_grid = (int)std::min<long long>((long long)b * r->fuse_sms, units);
             return issue_iteration(r, ctx->stream, nullptr) == ETCU_OK;
-        persist_smem = std::max(persist_smem, fuse_narrow(g.rx) ? fuse_narrow_smem_bytes(g.rx, g.rz, plan.ntaps)
-                                                                : fuse_smem_bytes(g.rx, g.rz, plan.ntaps));
         }, 2, &log);
         CK(ctx, cudaMemcpyAsync(vol->master, save, n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
         if (lowb) CK(ctx, cudaMemcpyAsync(vol->low, (char*)save + n * 4, lowb, cudaMemcpyDeviceToDevice, ctx->stream));
