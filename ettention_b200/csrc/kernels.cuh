@@ -1370,11 +1370,9 @@ __global__ void __launch_bounds__(kT, (kMulti ? 640 : 768) / kT) bp_block_kernel
             const bool in0 = x0 >= -kPad && x0 < a.W + kPad, in1 = x0 + 1 >= -kPad && x0 + 1 < a.W + kPad;
             const float2 p0 = in0 ? __ldg(r0 + x0) : zero, q0 = in1 ? __ldg(r0 + x0 + 1) : zero;
             const float2 p1 = in0 ? __ldg(r1 + x0) : zero, q1 = in1 ? __ldg(r1 + x0 + 1) : zero;
-            const float2 P0 =
-                make_float2(fadd(fmul(omb, p0.x), fmul(v.bw, p1.x)), fadd(fmul(omb, p0.y), fmul(v.bw, p1.y)));
-            const float2 P1 =
-                make_float2(fadd(fmul(omb, q0.x), fmul(v.bw, q1.x)), fadd(fmul(omb, q0.y), fmul(v.bw, q1.y)));
-            taps[e] = make_float4(fmul(P0.x, v.lamd), P0.y, fmul(fsub(P1.x, P0.x), v.lamd), fsub(P1.y, P0.y));
+            const float2 P0 = make_float2(fmaf(omb, p0.x, fmul(v.bw, p1.x)), fmaf(omb, p0.y, fmul(v.bw, p1.y)));
+            const float2 P1 = make_float2(fmaf(omb, q0.x, fmul(v.bw, q1.x)), fmaf(omb, q0.y, fmul(v.bw, q1.y)));
+            taps[e] = make_float4(fmul(P0.x, v.lamd), P0.y, fmul(P1.x, v.lamd), P1.y);
         }
     };
 
@@ -1410,13 +1408,14 @@ __global__ void __launch_bounds__(kT, (kMulti ? 640 : 768) / kT) bp_block_kernel
                     const float2 u = add2(add2(au, K2[j / 2]), m12);
                     const float2 f = __fadd2_rd(fma2(u, splat(256.f), splat(-127.5f)), splat(12582912.0f));
                     const uint32_t b0 = __float_as_uint(f.x), b1 = __float_as_uint(f.y);
-                    const float2 w = q8_weight2(f2(q8_k1(b0), q8_k1(b1)));
+                    const float2 k1 = f2(q8_k1(b0), q8_k1(b1));
+                    const float2 w = q8_weight2(k1), ow = fma2(k1, splat(-128.f), splat(129.f));  // a, 1 - a (exact)
                     const float4 t0 = *(const float4*)(bp_smem + (uint32_t)(tap0 + ((b0 >> 4) & 0xFFFFFFF0u)));
                     const float4 t1 = *(const float4*)(bp_smem + (uint32_t)(tap0 + ((b1 >> 4) & 0xFFFFFFF0u)));
-                    const float2 rl0 = fma2(splat(w.x), f2(t0.z, t0.w), f2(t0.x, t0.y));
-                    const float2 rl1 = fma2(splat(w.y), f2(t1.z, t1.w), f2(t1.x, t1.y));
+                    const float2 rl0 = fma2(splat(w.x), f2(t0.z, t0.w), mul2(splat(ow.x), f2(t0.x, t0.y)));
+                    const float2 rl1 = fma2(splat(w.y), f2(t1.z, t1.w), mul2(splat(ow.y), f2(t1.x, t1.y)));
                     // ParallelBeamsBackProjection.cl:40-50: r * lambda * d / L where L > eps
-                    const float c0 = fmul(rl0.x, rcp_approx(rl0.y)), c1 = fmul(rl1.x, rcp_approx(rl1.y));
+                    const float c0 = div_fast(rl0.x, rl0.y), c1 = div_fast(rl1.x, rl1.y);
                     const bool ok0 = rl0.y > kEps, ok1 = rl1.y > kEps;
                     if (kMulti) {
                         if (ok0) pv[j] = fadd(pv[j], c0);

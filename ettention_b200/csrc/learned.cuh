@@ -75,6 +75,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     return true;
 }
 
+// The same by every lane of a warp, with one outcome for all of them: a wait that gives up gives up
+// for the whole warp, so that no lane goes on alone.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+
 // ---------------------------------------------------------------- bulk copies (this GPU's memory only)
 __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2,
                                             int c3, int c4) {
@@ -114,13 +120,17 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 }
 
 // ---------------------------------------------------------------- tensor memory and MMA
+// Every lane executes these together (.aligned): each converges its warp first, whatever branches
+// the lanes took since the last one (a loop that stores for some lanes only, an elected lane's work).
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {  // one full warp
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
                  "r"(ncols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  // one full warp
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -143,6 +153,7 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 }
 // 16 consecutive 32-bit columns of this thread's lane (one full warp).
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
         "%15}, [%16];"
@@ -150,7 +161,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_ld() {
+    __syncwarp();
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
 
 // Shared-memory matrix descriptor, no swizzle (canonical "interleaved" layout: 8 rows of
 // 16 bytes form a core matrix).  lbo / sbo in bytes: for K-major operands lbo is the step
@@ -435,8 +449,7 @@ __global__ void __launch_bounds__(conv_threads<kLoad>(), 1) conv_tc_kernel(const
         int i = 0;
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++i) {
             const int acc = i & 1;
-            const bool got = mbar_wait(&accf[acc], (i >> 1) & 1);
-            __syncwarp();
+            const bool got = mbar_wait_warp(&accf[acc], (i >> 1) & 1);
             if (!got) {
                 if (lane == 0) atomicOr(a.err, kErrWaitDone);
                 break;
@@ -710,8 +723,7 @@ __global__ void __launch_bounds__(kZfoldThreads, 1) conv_zfold_kernel(const __gr
             const int x = xt * kTileX + m;
             for (int j = 0; j < len + 2; ++j, ++G) {
                 if (j < 2) continue;  // output z0 + j - 2 needs slices j - 2, j - 1, j
-                const bool got = mbar_wait(&accf[G & 3], (G >> 2) & 1);
-                __syncwarp();
+                const bool got = mbar_wait_warp(&accf[G & 3], (G >> 2) & 1);
                 if (!got) {
                     if (lane == 0) atomicOr(a.err, kErrWaitDone);
                     ok = false;
@@ -972,8 +984,8 @@ __global__ void __launch_bounds__(128) wgrad_tc_kernel(const __grid_constant__ C
         }
         if (ok) umma_commit(done);
     }
-    __syncwarp();
-    const bool got = mbar_wait(done, 0);
+    __syncwarp();  // the wait starts when the elected lanes are done
+    const bool got = mbar_wait_warp(done, 0);
     if (!got && threadIdx.x == 0) atomicOr(a.err, kErrWaitDone);
     __syncwarp();
     tc_fence_after();
