@@ -1270,16 +1270,22 @@ __global__ void __launch_bounds__(kBpColThreads, 4) bp_sart_column_kernel(const 
 // Per view (and sample) the two detector rows that row y projects to are blended once into
 // a shared-memory window of tap pairs over the columns that the brick projects to, the next
 // view's window while this one is applied; each voxel then takes one 16-byte shared load.
-// Coordinates, 1/256 weights and the update are those of bp_sart_column_kernel (two z voxels
-// per paired instruction), so results agree with bp_parallel_kernel's to a few ulps per update.
+// Coordinates and 1/256 weights are those of bp_sart_column_kernel (two z voxels per paired
+// instruction), so results agree with bp_parallel_kernel's to a few ulps per update.  It is no less exact
+// than that kernel: rows and taps are blended by weights (a difference of taps cancels where they differ by
+// their own size: 1.5e-7 for noise), the residual rows with lambda * chord in the weights, held in two
+// FP32 values.  That saves more roundings than the quotient by the reciprocal estimate costs with one
+// sample (error of an update against 64 bits 6.0e-8 .. 6.8e-8 in the 2-norm, 7.0e-8 .. 7.5e-8 there; with a Newton
+// step on the quotient the 12.1 ms below were 13.4), but not where the errors of several samples
+// average out, so those take the step (5.8e-8 and 6.0e-8 with 4 and 9 samples, 6.1e-8 and 6.2e-8 there).
 // Lanes hold consecutive x: their taps lie cos(tilt) entries apart, free of bank conflicts
 // without padding.
 // bp_parallel_kernel spends about 84 thread instructions per voxel and view (four 8-byte
-// gathers, the blend of four taps, an IEEE-accurate quotient): 38.2 ms for the 61 views of a
-// 1024 x 1024 x 256 SIRT iteration, 4.93 ms at 512 x 512 x 128.  This one takes 11.9 and 1.56 ms
-// and is bound by issue (about 14 instructions) and the shared-memory pipe (16 bytes per voxel
+// gathers, the blend of four taps, an IEEE-accurate quotient): 38.3 ms for the 61 views of a
+// 1024 x 1024 x 256 SIRT iteration, 4.93 ms at 512 x 512 x 128.  This one takes 12.1 and 1.60 ms
+// and is bound by issue (about 15 instructions) and the shared-memory pipe (16 bytes per voxel
 // and view, 7.3 ms at the former size) together.  With each thread forming the views' window
-// bounds and row weights itself instead of once per block it took 13.4 ms.
+// bounds and row weights itself instead of once per block it took 1.5 ms more.
 // kMulti: nsamples > 1, averaged over the samples with a ray length (used counts in bytes).
 struct BpBlockArgs {
     BpArgs a;
@@ -1291,9 +1297,12 @@ struct BpBlockArgs {
 // One view's (and sample's) constants for the block's brick, formed once.
 struct __align__(16) BpBlockView {
     float mu0, mu2, mu3, cy1;  // column coordinate: (mu0 (cx + sx) + cy1) + mu2 (cz + sz) + mu3
-    float sx, sz, bw, lamd;    // second detector row's weight, lambda * chord
+    float sx, sz;
+    float bw;                  // second detector row's weight
+    int x0lo;                  // first column of the window
+    float w0, w1, w0_lo, w1_lo;  // both rows' weights times lambda * chord: FP32 values and the rest of them
     long long row;             // element offset of the first detector row in the (residual, length) slots
-    int x0lo, pad;             // first column of the window
+    long long pad;
 };
 
 __host__ __device__ constexpr int bp_block_z(bool multi) { return multi ? 16 : 32; }
@@ -1337,7 +1346,6 @@ __global__ void __launch_bounds__(kT, (kMulti ? 640 : 768) / kT) bp_block_kernel
         v.mu3 = vc.mat[12];
         v.sx = s.x;
         v.sz = s.z;
-        v.lamd = fmul(a.lambda, s.w);
         const float py = fadd(cy, s.y);
         v.cy1 = fmul(vc.mat[4], py);
         // mat[1] is zero: every voxel of the row has the same detector row coordinate
@@ -1345,12 +1353,17 @@ __global__ void __launch_bounds__(kT, (kMulti ? 640 : 768) / kT) bp_block_kernel
         split_coord<kSampleQ8>(fadd(fadd(fmul(vc.mat[1], fadd(cxa, s.x)), fmul(vc.mat[5], py)), vc.mat[13]), a.H, y0,
                                v.bw);
         v.row = (long long)p * (long long)a.rl_slot + (long long)y0 * (long long)a.rl_pitch;
+        const float lamd = fmul(a.lambda, s.w), lamd_lo = fmaf(a.lambda, s.w, -lamd), omb = fsub(1.f, v.bw);
+        v.w0 = fmul(omb, lamd);
+        v.w1 = fmul(v.bw, lamd);
+        v.w0_lo = fmaf(omb, lamd_lo, fmaf(omb, lamd, -v.w0));
+        v.w1_lo = fmaf(v.bw, lamd_lo, fmaf(v.bw, lamd, -v.w1));
+        v.pad = 0;
         // the least column coordinate over the brick's corners (it is affine in x and z), with
         // two columns of margin for the float rounding
         const float lo = fminf(fmul(v.mu0, fadd(cxa, s.x)), fmul(v.mu0, fadd(cxb, s.x))) +
                          fminf(fmul(v.mu2, fadd(cza, s.z)), fmul(v.mu2, fadd(czb, s.z))) + v.cy1 + v.mu3;
         v.x0lo = (int)floorf(lo - 0.5f) - 2;
-        v.pad = 0;
         sv[i] = v;
     }
     auto stage = [&](int i) {
@@ -1370,9 +1383,11 @@ __global__ void __launch_bounds__(kT, (kMulti ? 640 : 768) / kT) bp_block_kernel
             const bool in0 = x0 >= -kPad && x0 < a.W + kPad, in1 = x0 + 1 >= -kPad && x0 + 1 < a.W + kPad;
             const float2 p0 = in0 ? __ldg(r0 + x0) : zero, q0 = in1 ? __ldg(r0 + x0 + 1) : zero;
             const float2 p1 = in0 ? __ldg(r1 + x0) : zero, q1 = in1 ? __ldg(r1 + x0 + 1) : zero;
-            const float2 P0 = make_float2(fmaf(omb, p0.x, fmul(v.bw, p1.x)), fmaf(omb, p0.y, fmul(v.bw, p1.y)));
-            const float2 P1 = make_float2(fmaf(omb, q0.x, fmul(v.bw, q1.x)), fmaf(omb, q0.y, fmul(v.bw, q1.y)));
-            taps[e] = make_float4(fmul(P0.x, v.lamd), P0.y, fmul(P1.x, v.lamd), P1.y);
+            auto residual = [&](float t0, float t1) {
+                return fmaf(v.w0, t0, fmaf(v.w1, t1, fmaf(v.w0_lo, t0, fmul(v.w1_lo, t1))));
+            };
+            taps[e] = make_float4(residual(p0.x, p1.x), fmaf(omb, p0.y, fmul(v.bw, p1.y)), residual(q0.x, q1.x),
+                                  fmaf(omb, q0.y, fmul(v.bw, q1.y)));
         }
     };
 
@@ -1415,7 +1430,8 @@ __global__ void __launch_bounds__(kT, (kMulti ? 640 : 768) / kT) bp_block_kernel
                     const float2 rl0 = fma2(splat(w.x), f2(t0.z, t0.w), mul2(splat(ow.x), f2(t0.x, t0.y)));
                     const float2 rl1 = fma2(splat(w.y), f2(t1.z, t1.w), mul2(splat(ow.y), f2(t1.x, t1.y)));
                     // ParallelBeamsBackProjection.cl:40-50: r * lambda * d / L where L > eps
-                    const float c0 = div_fast(rl0.x, rl0.y), c1 = div_fast(rl1.x, rl1.y);
+                    const float c0 = kMulti ? div_fast(rl0.x, rl0.y) : fmul(rl0.x, rcp_approx(rl0.y)),
+                                c1 = kMulti ? div_fast(rl1.x, rl1.y) : fmul(rl1.x, rcp_approx(rl1.y));
                     const bool ok0 = rl0.y > kEps, ok1 = rl1.y > kEps;
                     if (kMulti) {
                         if (ok0) pv[j] = fadd(pv[j], c0);

@@ -4,8 +4,7 @@ oracle: reconstructions of one block from a random start, so that the update of 
 is the sum over the block's views.
 
 The two kernels form the same coordinates and 1/256 weights; the staged one blends the two
-detector rows first and takes the reciprocal estimate of the ray length, a few ulps per
-view's contribution, so the updates agree to 1e-6 relative (SAME_TOL), and both with the
+detector rows first, a few ulps per view's contribution, so the updates agree to 1e-6 relative (SAME_TOL), and both with the
 FP32 oracle to the back-projection bar of 1e-4.  Shapes: rows of less than, exactly and one
 more than the 64 / 128 / 256 voxels of a block, odd sizes, slices that leave a block's last
 ones empty, detector rows between volume rows, a detector narrower than the volume's

@@ -8,8 +8,8 @@ edges of their tiles and of the rules that select them.
   below 128), each off by at most 1/256 of the two texels' difference, of the size of the values
   themselves: STEP_TOL = sqrt(1e-3) / 256 = 1.2e-4 relative.
 * bp_block_kernel for one view (rows that the column kernel does not take, from the size
-  at which they fill the chip) against bp_sart_row_kernel: the detector rows are blended first
-  and the ray length's reciprocal estimated, a few ulps per update: SAME_TOL.
+  at which they fill the chip) against bp_sart_row_kernel: the detector rows are blended first, a few
+  ulps per update: SAME_TOL.  Each one's own error is held to a 64-bit restatement.
 * the persistent fused SART step's narrow rows (several groups of threads on a chunk's
   slices) against the unfused kernels: bit-identical, widths around whole warps and the half
   block at which the wide form takes over.
@@ -151,6 +151,70 @@ def test_one_view_block_matches_row_kernel(ctxs, shape, tilt, half):
         assert O.rel_l2(outs[1], outs[0]) <= 1e-3
     else:
         assert O.rel_l2(outs[1] - init, outs[0] - init) <= SAME_TOL
+
+
+def _exact_update(shape, g, res, length, lam, samples):
+    """One view's update in 64 bits, at the kernels' coordinates and 1/256 weights: u and v step by
+    step in FP32 as both kernels form them, then the bilinear sums, the quotient and the samples' mean."""
+    f = np.float32
+    m = g.projection_matrix()
+    assert m[1] == 0 and m[9] == 0  # one detector row coordinate per y
+    centre = [f(-0.5 * n) + (np.arange(n, dtype=f) + f(0.5)) for n in shape]
+
+    def split(c, n):
+        t = c - f(0.5)
+        base = np.floor(t)
+        frac = np.floor((t - base) * f(256) + f(0.5)).astype(np.float64) / 256
+        return np.clip(base.astype(np.int64), -2, n) + 2, frac  # + 2: the padded images' offset
+    pad = [np.pad(a.astype(np.float64), 2) for a in (res, length)]
+    total, used = np.zeros(shape[::-1]), np.zeros(shape[::-1])
+    for s in g.sample_pattern([1, 1, 1], samples):
+        px, py, pz = (c + s[i] for i, c in enumerate(centre))
+        v0, b = split((m[1] * px[0] + m[5] * py) + m[13], res.shape[0])
+        rows = [a[v0] * (1 - b)[:, None] + a[v0 + 1] * b[:, None] for a in pad]
+        for z in range(shape[2]):
+            u = ((m[0] * px)[None, :] + (m[4] * py)[:, None] + m[8] * pz[z]) + m[12]
+            u0, a = split(u, res.shape[1])
+            R, L = (np.take_along_axis(r, u0, 1) * (1 - a) + np.take_along_axis(r, u0 + 1, 1) * a for r in rows)
+            total[z] += np.where(L > 1e-4, R * (float(f(lam)) * float(s[3])) / np.maximum(L, 1e-4), 0.0)
+            used[z] += L > 1e-4
+    return total / np.maximum(used, 1)
+
+
+@pytest.mark.parametrize("shape,tilt,smooth,samples", [((1001, 61, 64), -27.5, False, 1), ((999, 64, 63), 48.0, False, 1),
+                                                       ((501, 91, 91), 0.0, False, 1), ((501, 91, 91), 69.0, False, 1),
+                                                       ((1001, 61, 64), -27.5, True, 1), ((501, 91, 91), 61.5, True, 1),
+                                                       ((130, 64, 65), -35.0, False, 4), ((130, 64, 65), 20.0, True, 9)])
+def test_staged_update_is_as_close_to_64_bits_as_the_general_kernels(ctxs, shape, tilt, smooth, samples):
+    """bp_block_kernel's FP32 error per update is no larger than that of bp_sart_row_kernel (one sample) and
+    bp_parallel_kernel (several), in the 2-norm and in the largest error, for noise residuals and ray
+    lengths (taps that differ by their own size) and for smooth ones."""
+    import torch
+    from ettention_b200.operators import BackProjectionOperator, GPUMappedVolume, mrc_base_geometry
+    X, Y, Z = shape
+    rng = np.random.Generator(np.random.PCG64(X + Y))
+    g = mrc_base_geometry(X, Y).rotated(tilt)
+    if smooth:
+        x, y = np.meshgrid(np.arange(X) / 17.0, np.arange(Y) / 13.0)
+        res, length = np.sin(x) * np.cos(y) + 0.3, Z * (1.2 + 0.2 * np.sin(0.3 * x))
+    else:
+        res, length = rng.normal(size=(Y, X)), rng.uniform(0.5, 2.0 * Z, size=(Y, X))
+    res, length = res.astype(np.float32), length.astype(np.float32)
+    exact = _exact_update(shape, g, res, length, 0.3, samples)
+    errors = []
+    for ctx in ctxs:
+        vol = GPUMappedVolume(ctx, shape)
+        vol.upload(np.zeros((Z, Y, X), np.float32))
+        bp = BackProjectionOperator(vol, 0.3, samples)
+        bp.setScannerGeometry(g)
+        bp.setInput(torch.tensor(res, device="cuda"), torch.tensor(length, device="cuda"), 1)
+        bp.execute()
+        d = vol.download().astype(np.float64) - exact
+        errors.append((np.linalg.norm(d) / np.linalg.norm(exact), np.abs(d).max() / np.sqrt((exact ** 2).mean())))
+        vol.close()
+    assert errors[0][0] < 2e-7  # the 64-bit restatement takes the kernels' taps
+    assert errors[1][0] <= errors[0][0]
+    assert errors[1][1] <= 1.1 * errors[0][1]  # the extreme of some 10^5 .. 10^6 updates
 
 
 @pytest.mark.parametrize("shape", [(4, 5, 3), (60, 9, 70), (64, 6, 64), (68, 12, 130), (256, 7, 9), (260, 5, 33),
