@@ -102,3 +102,38 @@ def rel_l2(a, b) -> float:
     b = np.asarray(b, np.float64)
     nb = np.linalg.norm(b.ravel())
     return float(np.linalg.norm((a - b).ravel()) / (nb if nb > 0 else 1.0))
+
+
+def _recorded_kernels(run, pad: float) -> list:
+    """Names of the GPU activity records while run() runs, one per launch.  The profiler keeps what lies
+    between its start and its stop on the host's clock, and the records carry the GPU's: `pad` seconds on
+    both sides keep a region of some microseconds away from those ends."""
+    import time
+
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        time.sleep(pad)
+        run()
+        torch.cuda.synchronize()
+        time.sleep(pad)
+    return [e.name for e in prof.events()]
+
+
+def launched_back_projectors(run, count: int, record=_recorded_kernels, attempts: int = 4):
+    """The names of the `count` back-projection kernels that run() launches, or None when no attempt's
+    records held all of them: records may be missing, and an incomplete list says nothing about which
+    kernels ran.  run() may be called several times and has to start from the same state each time."""
+    for k in range(attempts):
+        names = [n for n in record(run, 0.01 * 3 ** k) if "bp_" in n]
+        if len(names) == count:
+            return set(names)
+    return None
+
+
+def require_records(*names) -> None:
+    """Skips the rest of a test (the route; its results have been compared) without complete records."""
+    import pytest
+    if any(n is None for n in names):
+        pytest.skip("the GPU's activity records stayed incomplete")

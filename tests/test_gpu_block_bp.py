@@ -14,6 +14,8 @@ import os
 import numpy as np
 import pytest
 
+from tests.helpers import launched_back_projectors, require_records
+
 pytestmark = pytest.mark.gpu
 
 BP_TOL = 1e-4
@@ -53,8 +55,6 @@ CASES = [
 
 @pytest.mark.parametrize("shape,nviews,vpitch,width,subs,samples,storage", CASES)
 def test_staged_block_matches_general_and_oracle(ctxs, shape, nviews, vpitch, width, subs, samples, storage):
-    import torch
-    from torch.profiler import ProfilerActivity, profile
     from oracle import oracle as O
     from ettention_b200 import _abi
     from ettention_b200.operators import (AlgebraicParameterSet, BlockIterativeReconstructionOperator,
@@ -77,27 +77,28 @@ def test_staged_block_matches_general_and_oracle(ctxs, shape, nviews, vpitch, wi
     outs, names = [], []
     for ctx in ctxs:
         vol = GPUMappedVolume(ctx, shape, voxel_type=kind, subvolume_count=subs)
-        vol.upload(init)
         rec = BlockIterativeReconstructionOperator(vol, geoms, projs, p, use_graph=False)
-        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+
+        def run():
+            vol.upload(init)
             rec.runNiterations(1)
-            torch.cuda.synchronize()
-        names.append({e.name for e in prof.events()})
+        names.append(launched_back_projectors(run, subs))
         outs.append(rec.getReconstructedVolume())
         rec.close()
         vol.close()
-    assert any("bp_parallel_kernel" in n for n in names[0]) and not any("bp_block_kernel" in n for n in names[0])
-    assert any("bp_block_kernel" in n for n in names[1]) and not any("bp_parallel_kernel" in n for n in names[1])
     assert np.abs(outs[0] - init).max() > 0
     if storage == "half":  # re-rounded after every view: a last-bit difference can move a voxel by one half ulp
         assert O.rel_l2(outs[1], outs[0]) <= 1e-3
-        return
-    # a pixel whose true ray length is near the 1e-4 threshold would be kept by one kernel and skipped by the
-    # other: random projections leave none here
-    assert O.rel_l2(outs[1] - init, outs[0] - init) <= SAME_TOL
+    else:
+        # a pixel whose true ray length is near the 1e-4 threshold would be kept by one kernel and skipped by the
+        # other: random projections leave none here
+        assert O.rel_l2(outs[1] - init, outs[0] - init) <= SAME_TOL
     if storage == "float32":
         setup = O.ReconstructionSetup(O.VolumeGeometry.centered(shape, subvolumes=subs),
                                       [oracle_geometry(g) for g in geoms], projs, 0.3, nviews, 1, samples)
         vo = init.copy()
         O.block_iterative(setup, vo, 1, 32)
         assert O.rel_l2(outs[1] - init, vo - init) <= BP_TOL
+    require_records(*names)
+    assert all("bp_parallel_kernel" in n for n in names[0])
+    assert all("bp_block_kernel" in n for n in names[1])
