@@ -618,18 +618,36 @@ void launch_bp_block(const BpArgs& a, const BpBlockPlan& p, etcu_voxel_type t, i
               : launch_bp_block_s<64, false>(b, grid, smem, t, device, st);
 }
 
-// Whether bp_persp_row_kernel applies to `n` perspective views of a sub-volume: 1/256 sampling,
-// one sample per voxel, no mask, no detector column or depth that depends on y, and a source
-// outside the sub-volume along some axis.  It forms about half the instructions per voxel of
-// bp_perspective_kernel, whose chunks run along z, so it is the faster one unless its last
-// 16-voxel chunk in y leaves more than a third of the work idle.
+// Whether bp_persp_row_kernel applies to the views of a sub-volume: 1/256 sampling, one sample per
+// voxel, no mask, no detector column or depth that depends on y, and a source outside the sub-volume
+// along some axis.  Both kernels take rounds of blocks over the chip, and each does the work of its
+// padding too: 16 y by 4 z here, 16 z by 8 y in bp_perspective_kernel.  That kernel's time over this one's,
+// 64 .. 512 x 15 .. 400 x 16 .. 160 voxels:
+//  - all blocks resident together: 1.05 .. 1.5 whatever the padding; one view on a volume with 16-bit voxels
+//    (8 along x are half a sector of those) 1.01 .. 1.2 up to half of the residency, 0.97 at all of it;
+//  - one view beyond that has little work per block: FP32 0.81 .. 1.2 in the second round, half empty, and
+//    1.00 .. 1.25 from one and a half rounds with padding at most a tenth above the other's; 16-bit
+//    0.76 .. 1.2;
+//  - two or three views with that padding: FP32 1.03 .. 1.7; 16-bit 1.02 .. 1.5 from one and a half rounds, 0.95
+//    before; with more padding down to 0.85;
+//  - four or more: 1.07 .. 1.5 with padding up to a quarter above the other's; 0.90 .. 1.06 with a third.
 bool plan_bp_persp_rows(const etcu_volume* vol, const BpArgs& a, etcu_sampling sm, const ViewConst* hvc,
                         const uint32_t* vids) {
     const SlabConst& g = a.slab;
     if (!vol->ctx->bp_column || sm != ETCU_SAMPLING_Q8 || a.mask || a.persp_n != 1) return false;
-    const int chunks = (g.ry + kBpYPersp - 1) / kBpYPersp;
-    if (chunks > 65535 || (g.rx + 31) / 32 > 65535 || 3ll * chunks * kBpYPersp > 4ll * g.ry)
-        return false;
+    const long long chunks = (g.ry + kBpYPersp - 1) / kBpYPersp, zt = (g.rz + 3) / 4,
+                    xt = (g.rx + 8 * kBpRowWarps - 1) / (8 * kBpRowWarps);
+    if (chunks > 65535 || xt > 65535) return false;
+    const long long blocks = chunks * zt * xt, resident = (long long)kBpRowBlocks * device_sms(vol->ctx->device);
+    const bool fp32 = vol->type == ETCU_VOXEL_FLOAT32, few = a.nviews < 4;
+    if (blocks > (a.nviews == 1 && !fp32 ? resident / 2 : resident)) {
+        if (a.nviews == 1 && !fp32) return false;
+        if (few && !(fp32 && a.nviews > 1) && 2 * blocks < 3 * resident) return false;
+        // padded voxels of one x column, here and there
+        const long long own = chunks * kBpYPersp * zt * 4;
+        const long long other = (long long)((g.rz + kBpZPersp - 1) / kBpZPersp) * kBpZPersp * ((g.ry + 7) / 8) * 8;
+        if (few ? 10 * own > 11 * other : 4 * own > 5 * other) return false;
+    }
     if (!(g.vs.x >= 1e-6f && g.vs.y >= 1e-6f && g.vs.z >= 1e-6f)) return false;
     for (int i = 0; i < a.nviews; ++i) {
         const ViewConst& c = hvc[vids ? vids[i] : 0];

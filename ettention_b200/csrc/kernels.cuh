@@ -2368,6 +2368,7 @@ __global__ void __launch_bounds__(256, 4) bp_perspective_kernel(const __grid_con
 // step (about one in a thousand), where a last bit decides the weight.
 constexpr int kBpYPersp = 16;
 constexpr int kBpRowWarps = 4;  // per block of 8 * kBpRowWarps x by 4 z, side by side along x
+constexpr int kBpRowBlocks = 24 / kBpRowWarps;  // resident blocks per multiprocessor (80 registers a thread)
 
 __host__ __device__ constexpr size_t bp_persp_row_smem_bytes(int nviews) {
     return ((size_t)nviews * sizeof(BpView) + 15) / 16 * 16 + (size_t)nviews * (kBpYPersp / 2) * (16 + 8);
@@ -2380,7 +2381,7 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 }
 
 template <int kStore, bool kClamp>
-__global__ void __launch_bounds__(32 * kBpRowWarps, 24 / kBpRowWarps) bp_persp_row_kernel(const __grid_constant__ BpArgs a) {
+__global__ void __launch_bounds__(32 * kBpRowWarps, kBpRowBlocks) bp_persp_row_kernel(const __grid_constant__ BpArgs a) {
     extern __shared__ __align__(16) unsigned char bp_smem[];
     BpView* sv = (BpView*)bp_smem;
     bp_stage(a, sv, nullptr, false);

@@ -51,21 +51,28 @@ def ctxs():
 
 
 PERSP = [
-    # (X, Y, Z), views, detector (W, H) or None, sign of the row pitch, source distance / X, clamp, sub-volumes, storage
-    ((32, 16, 4), 3, None, 1, 10.0, None, 1, "float32"),
-    ((33, 15, 5), 4, None, 1, 10.0, None, 1, "float32"),
-    ((70, 31, 9), 5, None, -1, 10.0, None, 2, "float32"),
-    ((100, 48, 37), 7, (60, 20), 1, 3.0, None, 1, "float32"),   # most voxels project off the detector
-    ((64, 32, 20), 1, None, 1, 10.0, (0.1, 0.9), 1, "float32"),
-    ((96, 30, 24), 8, None, 1, 10.0, None, 3, "bf16_master"),
-    ((96, 30, 24), 3, None, 1, 10.0, None, 1, "f16_master"),
-    ((96, 30, 24), 3, None, 1, 10.0, None, 1, "half"),
-    ((32, 17, 8), 2, None, 1, 10.0, None, 1, "float32"),        # too many idle rows: the general kernel
+    # (X, Y, Z), views, detector (W, H) or None, sign of the row pitch, source distance / X, clamp, sub-volumes, storage,
+    # whether the row kernel takes it
+    ((32, 16, 4), 3, None, 1, 10.0, None, 1, "float32", True),
+    ((33, 15, 5), 4, None, 1, 10.0, None, 1, "float32", True),
+    ((70, 31, 9), 5, None, -1, 10.0, None, 2, "float32", True),
+    ((100, 48, 37), 7, (60, 20), 1, 3.0, None, 1, "float32", True),   # most voxels project off the detector
+    ((64, 32, 20), 1, None, 1, 10.0, (0.1, 0.9), 1, "float32", True),
+    ((96, 30, 24), 8, None, 1, 10.0, None, 3, "bf16_master", True),
+    ((96, 30, 24), 3, None, 1, 10.0, None, 1, "f16_master", True),
+    ((96, 30, 24), 3, None, 1, 10.0, None, 1, "half", True),
+    ((32, 17, 8), 2, None, 1, 10.0, None, 1, "float32", True),        # mostly padding, but resident
+    ((256, 129, 56), 1, None, 1, 10.0, None, 1, "float32", False),    # one view, the second round of blocks half empty
+    ((256, 129, 56), 2, None, 1, 10.0, None, 1, "float32", True),
+    ((256, 64, 64), 1, None, 1, 10.0, None, 1, "bf16_master", False),  # one view, more than half of the residency
+    ((256, 129, 56), 2, None, 1, 10.0, None, 1, "bf16_master", False),
+    ((256, 17, 224), 2, None, 1, 10.0, None, 1, "float32", False),    # a third more padding than along z
+    ((256, 129, 56), 4, None, 1, 10.0, None, 1, "half", True),
 ]
 
 
-@pytest.mark.parametrize("shape,nviews,det,sign,dist,clamp,subs,storage", PERSP)
-def test_perspective_rows_match_general(ctxs, shape, nviews, det, sign, dist, clamp, subs, storage):
+@pytest.mark.parametrize("shape,nviews,det,sign,dist,clamp,subs,storage,rows", PERSP)
+def test_perspective_rows_match_general(ctxs, shape, nviews, det, sign, dist, clamp, subs, storage, rows):
     from oracle import oracle as O
     from ettention_b200 import _abi
     from ettention_b200.operators import (AlgebraicParameterSet, BlockIterativeReconstructionOperator,
@@ -106,7 +113,7 @@ def test_perspective_rows_match_general(ctxs, shape, nviews, det, sign, dist, cl
         assert (np.abs(update - general).max(axis=1) > 1e-6 * np.abs(general).max()).mean() <= 1e-2  # columns along y
     require_records(*names)
     assert not any("bp_persp_row_kernel" in n for n in names[0])
-    assert any("bp_persp_row_kernel" in n for n in names[1]) == (shape != (32, 17, 8))
+    assert any("bp_persp_row_kernel" in n for n in names[1]) == rows
 
 
 @pytest.mark.parametrize("shape,det,sign,dist,subs", [((32, 16, 4), None, 1, 10.0, 1), ((33, 15, 5), None, 1, 10.0, 1),
