@@ -584,6 +584,20 @@ bool plan_bp_block(const etcu_volume* vol, const SlabConst& g, const ViewConst* 
     return p.ntaps <= 1024;
 }
 
+// Whether one view that the column kernel does not take (x no multiple of 4) goes to the window-staged
+// kernel rather than to bp_sart_row_kernel.  One view does not repay a window's set-up on a small volume
+// or many idle lanes: from the size at which the blocks fill the chip with 32 slices per thread, and
+// padding of at most three quarters of the voxels, it is 1.08 .. 1.7 times as fast on FP32 volumes and
+// 1.04 .. 1.5 with a 16-bit copy (65 .. 513 x 64 .. 600 x 36 .. 192 voxels; 501 x 363 x 179: 100 -> 65 us);
+// with twice the voxels or more 0.95 .. 1.06.  Half volumes stay with the row kernel (0.66 .. 1.1 of its speed here).
+bool one_view_block_pays(const etcu_volume* vol, const SlabConst& g, const BpBlockPlan& p) {
+    if (vol->type == ETCU_VOXEL_HALF16) return false;
+    const long long voxels = (long long)g.rx * g.ry * g.rz;
+    const long long padded = (long long)((g.rx + p.threads - 1) / p.threads) * p.threads *
+                             ((g.rz + p.zper - 1) / p.zper) * p.zper * g.ry;
+    return voxels >= 32ll * 768 * device_sms(vol->ctx->device) && 4 * padded <= 7 * voxels;
+}
+
 template <int kT, bool kMulti>
 void launch_bp_block_s(const BpBlockArgs& b, dim3 grid, size_t smem, etcu_voxel_type t, int device, cudaStream_t st) {
     static std::atomic<unsigned long long> opted{0};
@@ -707,12 +721,9 @@ uint32_t launch_bp(const etcu_volume* vol, const BpArgs& a0, bool persp, etcu_sa
             launch_bp_col(a0, plan, st);
             return 1;
         }
-        // rows that the column kernel does not take (x no multiple of 4, 16-bit volumes), from
-        // the size at which they fill the chip with 32 slices per thread (501 x 363 x 179: 129 -> 92 us;
-        // smaller volumes leave the window's set-up exposed)
         BpBlockPlan one;
-        if (sm == ETCU_SAMPLING_Q8 &&
-            (long long)a0.slab.rx * a0.slab.ry * a0.slab.rz >= 32ll * 768 * device_sms(dev) && plan_bp_block(vol, a0.slab, hvc, hsmp, 1, vids, 1, one)) {
+        if (sm == ETCU_SAMPLING_Q8 && plan_bp_block(vol, a0.slab, hvc, hsmp, 1, vids, 1, one) &&
+            one_view_block_pays(vol, a0.slab, one)) {
             launch_bp_block(a0, one, vol->type, dev, st);
             return 1;
         }

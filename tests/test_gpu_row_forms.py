@@ -162,14 +162,18 @@ def test_perspective_rows_match_oracle(ctxs, shape, det, sign, dist, subs):
         assert all("bp_persp_row_kernel" in n for n in names)
 
 
-@pytest.mark.parametrize("shape,tilt,half", [((1001, 61, 64), -27.5, False), ((1999, 33, 57), 63.0, False),
-                                             ((256, 240, 61), 41.0, True)])
-def test_one_view_block_matches_row_kernel(ctxs, shape, tilt, half):
+@pytest.mark.parametrize("shape,tilt,storage,block", [((1001, 61, 64), -27.5, "float32", True),
+                                                       ((1999, 33, 57), 63.0, "float32", True),
+                                                       ((255, 240, 61), 41.0, "bf16_master", True),
+                                                       ((256, 240, 61), 41.0, "half", False),
+                                                       ((129, 601, 68), 41.0, "float32", False)])  # half of it padding
+def test_one_view_block_matches_row_kernel(ctxs, shape, tilt, storage, block):
     import torch
     from oracle import oracle as O
     from ettention_b200 import _abi
     from ettention_b200.operators import BackProjectionOperator, GPUMappedVolume, mrc_base_geometry
     X, Y, Z = shape
+    kind = {"float32": _abi.VOXEL_FLOAT32, "bf16_master": _abi.VOXEL_BF16_MASTER, "half": _abi.VOXEL_HALF16}[storage]
     rng = np.random.Generator(np.random.PCG64(X))
     g = mrc_base_geometry(X, Y).rotated(tilt)
     res = torch.tensor(rng.normal(size=(Y, X)).astype(np.float32), device="cuda")
@@ -177,7 +181,7 @@ def test_one_view_block_matches_row_kernel(ctxs, shape, tilt, half):
     init = rng.uniform(0.0, 1.0, size=(Z, Y, X)).astype(np.float32)
     outs, names = [], []
     for ctx in ctxs:
-        vol = GPUMappedVolume(ctx, shape, voxel_type=_abi.VOXEL_HALF16 if half else _abi.VOXEL_FLOAT32)
+        vol = GPUMappedVolume(ctx, shape, voxel_type=kind)
         bp = BackProjectionOperator(vol, 0.3, 1)
         bp.setScannerGeometry(g)
         bp.setInput(res, length, 1)
@@ -189,13 +193,13 @@ def test_one_view_block_matches_row_kernel(ctxs, shape, tilt, half):
         outs.append(vol.download())
         vol.close()
     assert np.abs(outs[0] - init).max() > 0
-    if half:
-        assert O.rel_l2(outs[1], outs[0]) <= 1e-3
-    else:
+    if block:
         assert O.rel_l2(outs[1] - init, outs[0] - init) <= SAME_TOL
+    else:
+        assert np.array_equal(outs[1], outs[0])
     require_records(*names)
     assert any("bp_sart_row_kernel" in n for n in names[0])
-    assert any("bp_block_kernel" in n for n in names[1])
+    assert any("bp_block_kernel" in n for n in names[1]) == block
 
 
 def _exact_update(shape, g, res, length, lam, samples):
