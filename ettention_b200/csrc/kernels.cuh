@@ -1515,11 +1515,13 @@ __host__ __device__ constexpr size_t fuse_smem_bytes(int rx, int rz, int ntaps) 
 
 // Narrow rows (kNarrow): with two voxels of a row per thread, a 128-voxel row would occupy 64 of the
 // 512 threads and a chunk's eight slices be updated one after the other, once per 1 KB of volume and
-// barrier.  Rows of at most half the block instead put 512 / (rx / 2, in whole warps) groups of
+// barrier.  Rows of at most 256 voxels instead put 512 / (rx / 2, in whole warps) groups of
 // threads on different slices of a chunk, and a chunk holds as many slices as 16 KB do.
 // (128 x 128 x 64 over 61 views, five iterations: 5.60 -> 3.87 ms; a step there is a chain of
-// fetch, update and walk in one block per row, not work.)
-__host__ __device__ constexpr bool fuse_narrow(int rx) { return rx <= kFuseThreads; }
+// fetch, update and walk in one block per row, not work.)  Times of the wide form over the narrow one's, 64 .. 600
+// rows of 40 .. 128 slices: 64 voxels 1.53 .. 2.1, 128 1.31 .. 1.6, 256 1.03 .. 1.14; 288 .. 512, which leave two or
+// three groups and chunks of eight slices, 0.74 .. 0.97.
+__host__ __device__ constexpr bool fuse_narrow(int rx) { return rx <= kFuseThreads / 2; }
 __host__ __device__ constexpr int fuse_narrow_chunk(int rx) {
     return 4096 / rx / 8 * 8 < kFuseZc ? kFuseZc : (4096 / rx / 8 * 8 > 64 ? 64 : 4096 / rx / 8 * 8);
 }
