@@ -273,13 +273,27 @@ size_t slab_offset_elems(const etcu_volume* vol, const SlabConst& s) {
 }
 
 // ------------------------------------------------------------- launches
+// Several views: one after the other, or all views of a detector row together (their rays cross the
+// same few volume rows, which then stay in L2).  Together pays from about the size of the L2: 1.04 .. 1.15 times
+// as fast from 100 MB of voxels on (2 .. 41 views of 512 x 500 x 100 .. 1500 x 1500 x 200; 61 views of
+// 1024 x 1024 x 256: 17.5 -> 15.7 ms), no gain and down to 0.80 below 54 MB, where the last blocks of the
+// launch are then full-length rays of every view (8 views of 250 x 60 x 64: 16.2 -> 20.3 us).
+constexpr size_t kFpBesideBytes = 80u << 20;
+
 template <typename VoxT, bool kMask, int kPath>
-void launch_fp_t(const FpArgs& a, uint32_t nviews, cudaStream_t st) {
-    dim3 block(128);
-    dim3 grid;
-    if (kPath == kFpPathPerspective) grid = dim3((a.W + 15) / 16 * nviews, (a.H + 7) / 8);
-    else grid = dim3((a.W + 127) / 128 * nviews, a.H);
-    forward_project_kernel<VoxT, kMask, kPath><<<grid, block, 0, st>>>(a);
+void launch_fp_t(const FpArgs& a0, uint32_t nviews, cudaStream_t st) {
+    constexpr bool kPersp = kPath == kFpPathPerspective;
+    const unsigned tiles = kPersp ? (a0.W + 15) / 16 : (a0.W + 127) / 128, rows = kPersp ? (a0.H + 7) / 8 : a0.H;
+    const size_t bytes = (size_t)a0.slab.rx * a0.slab.ry * a0.slab.rz * sizeof(VoxT);
+    FpArgs a = a0;
+    a.beside = nviews > 1 && bytes >= kFpBesideBytes ? 1 : 0;
+    for (uint32_t done = 0; done < nviews; done += 65535) {
+        const unsigned n = std::min(nviews - done, 65535u);
+        a.first = a0.first + done;
+        if (a0.rl) a.rl = a0.rl + (size_t)done * a0.rl_slot;
+        const dim3 grid = a.beside ? dim3(tiles, n, rows) : dim3(tiles, rows, n);
+        forward_project_kernel<VoxT, kMask, kPath><<<grid, 128, 0, st>>>(a);
+    }
 }
 
 template <typename VoxT, bool kMask>

@@ -399,7 +399,8 @@ struct FpArgs {
     const ViewConst* views;     // device view table (nullptr: use inline_view)
     ViewConst inline_view;
     const uint32_t* order;      // iteration order (view ids), may be nullptr
-    uint32_t first;             // order position of grid.z == 0
+    uint32_t first;             // order position of the launch's first view
+    int beside;                 // the launch's views: 0 in blockIdx.z, 1 in blockIdx.y (detector rows in the other)
     int W, H, samples;
     int mode, overwrite, loc;
     float* out_v;               // mode 0
@@ -533,13 +534,8 @@ template <typename VoxT, bool kMask, int kPath>
 __global__ void __launch_bounds__(128, (kPath == kFpPathXz || kPath == kFpPathXzNoCap) ? 7
                                            : (kPath == kFpPathPerspective ? 8 : 4))
     forward_project_kernel(const __grid_constant__ FpArgs a) {
-    // grid: (tiles of a detector row x views, detector rows): the views of one detector row
-    // run together, since their rays cross the same few volume rows, which then stay in L2
-    // (61 views of 1024 x 1024 x 256: 17.5 -> 15.7 ms; blocks of eight perspective views at
-    // 2048 x 2048 x 512, 31 views: 81.2 -> 76.3 ms)
-    const int tiles = kPath == kFpPathPerspective ? (a.W + 15) / 16 : (a.W + 127) / 128;
-    const int p = (int)blockIdx.x / tiles;
-    fp_pixel<VoxT, kMask, kPath>(a, a.first, p, (int)blockIdx.x - p * tiles, (int)blockIdx.y);
+    const int v = a.beside ? (int)blockIdx.y : (int)blockIdx.z, row = a.beside ? (int)blockIdx.z : (int)blockIdx.y;
+    fp_pixel<VoxT, kMask, kPath>(a, a.first, v, (int)blockIdx.x, row);
 }
 
 // Batched tilt series: series s = blockIdx.z reads its arguments from table[s]

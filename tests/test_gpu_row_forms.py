@@ -10,6 +10,7 @@ edges of their tiles and of the rules that select them.
 * bp_block_kernel for one view (rows that the column kernel does not take, from the size
   at which they fill the chip) against bp_sart_row_kernel: the detector rows are blended first, a few
   ulps per update: SAME_TOL.  Each one's own error is held to a 64-bit restatement.
+* several views of one launch side by side against each view in a launch of its own.
 * the persistent fused SART step's narrow rows (several groups of threads on a chunk's
   slices) against the unfused kernels: bit-identical, widths around whole warps and the half
   block at which the wide form takes over.
@@ -295,6 +296,39 @@ def test_narrow_fused_rows_are_bit_identical_to_unfused(shape, storage):
     assert np.abs(outs[0][0] - init).max() > 0
     assert np.array_equal(outs[1][0], outs[0][0])
     assert outs[1][1] == pytest.approx(outs[0][1], rel=1e-12)
+
+
+@pytest.mark.parametrize("perspective", [False, True])
+def test_views_side_by_side_write_their_own_images(ctxs, perspective):
+    """A volume of 92 MB, whose views share a launch's detector rows: the sum of the squared residuals
+    over 3 views equals the sum over a launch per view (the same FP32 values, sums in FP64)."""
+    from ettention_b200 import _abi
+    from ettention_b200.operators import (AlgebraicParameterSet, BlockIterativeReconstructionOperator,
+                                          GPUMappedVolume, ScannerGeometry)
+    X, Y, Z, W, H = 300, 300, 256, 291, 77
+    if perspective:
+        base = ScannerGeometry([0.0, 0.0, 10.0 * X], [-0.55 * X, -0.55 * Y, -float(X)], [1.1 * X / W, 0.0, 0.0],
+                               [0.0, 1.1 * Y / H, 0.0], W, H, True)
+    else:
+        base = ScannerGeometry([-0.5 * X, -0.5 * Y, float(X)], [-0.5 * X, -0.5 * Y, -float(X)], [X / W, 0.0, 0.0],
+                               [0.0, Y / H, 0.0], W, H, False)
+    geoms = [base.rotated(a) for a in (-50.0, 3.0, 41.0)]
+    rng = np.random.Generator(np.random.PCG64(3))
+    projs = (rng.uniform(0.0, 4.0, size=(3, H, W)) * np.array([1.0, 8.0, 64.0])[:, None, None]).astype(np.float32)
+    vol = GPUMappedVolume(ctxs[1], (X, Y, Z))
+    vol.upload(rng.uniform(0.0, 1.0, size=(Z, Y, X)).astype(np.float32))
+
+    def residual(views):
+        p = AlgebraicParameterSet(algorithm="sirt", block_size=_abi.BLOCK_ALL, iterations=1, lam=0.3,
+                                  order=_abi.ORDER_IDENTITY)
+        rec = BlockIterativeReconstructionOperator(vol, [geoms[v] for v in views], projs[views], p, use_graph=False)
+        r = rec.data_residual_sq()
+        rec.close()
+        return r
+    together, apart = residual([0, 1, 2]), [residual([v]) for v in range(3)]
+    vol.close()
+    assert all(a > 0 for a in apart)
+    assert together == pytest.approx(sum(apart), rel=1e-12)
 
 
 @pytest.mark.parametrize("res,batch", [((4, 4, 4), 2), ((124, 12, 36), 1), ((264, 4, 68), 2)])
