@@ -402,6 +402,28 @@ void launch_bp_sart_m(const BpArgs& a, etcu_voxel_type t, etcu_sampling sm, cuda
     }
 }
 
+// Whether every voxel centre of a sub-volume lies inside a tap window that the host bounds with two columns
+// of margin: |256 u| < 2^22 for the tap split, and terms of u below 2^20, so that the FP32 roundings of the
+// sums (half an ulp, 2^-4, for each of about eight) stay within half a column.  A box millions of
+// pixels from the origin has coordinates too coarse for that.
+bool tap_window_holds(const SlabConst& g, const ViewConst& c, const float4& s, double& umin, double& umax) {
+    umin = 1e300;
+    umax = -1e300;
+    double largest = 0.0;
+    for (int q = 0; q < 8; ++q) {
+        const double x = (q & 1) ? g.rx - 1 : 0, y = (q & 2) ? g.ry - 1 : 0, z = (q & 4) ? g.rz - 1 : 0;
+        const double tx = (double)c.mat[0] * ((double)g.bmin.x + (x + 0.5) * g.vs.x + s.x);
+        const double ty = (double)c.mat[4] * ((double)g.bmin.y + (y + 0.5) * g.vs.y + s.y);
+        const double tz = (double)c.mat[8] * ((double)g.bmin.z + (z + 0.5) * g.vs.z + s.z);
+        const double u = tx + ty + tz + c.mat[12];
+        if (!(u > -16000.0 && u < 16000.0)) return false;  // NaN too
+        umin = std::min(umin, u);
+        umax = std::max(umax, u);
+        largest = std::max(largest, std::fabs(tx) + std::fabs(ty) + std::fabs(tz) + std::fabs((double)c.mat[12]));
+    }
+    return largest < 1048576.0;
+}
+
 struct BpColPlan {
     int groups = 0;  // 4-voxel x groups per thread (1 or 2)
     int shadow = 0;  // the master's 16-bit shadow written beside it (1: FP16, 2: BF16)
@@ -464,17 +486,8 @@ bool plan_bp_col(const etcu_volume* vol, const SlabConst& g, const ViewConst& vc
     if (!ctx->bp_column || vol->type == ETCU_VOXEL_HALF16 || vol->mask) return false;
     p.shadow = vol->type == ETCU_VOXEL_F16_MASTER ? 1 : (vol->type == ETCU_VOXEL_BF16_MASTER ? 2 : 0);
     if (g.rx <= 0 || g.ry <= 0 || g.rz <= 0 || g.rx % 4 != 0 || g.rx > 8 * kBpColThreads) return false;
-    double umin = 1e300, umax = -1e300;
-    for (int c = 0; c < 8; ++c) {
-        const double x = (c & 1) ? g.rx - 1 : 0, y = (c & 2) ? g.ry - 1 : 0, z = (c & 4) ? g.rz - 1 : 0;
-        const double px = (double)g.bmin.x + (x + 0.5) * g.vs.x + smp.x;
-        const double py = (double)g.bmin.y + (y + 0.5) * g.vs.y + smp.y;
-        const double pz = (double)g.bmin.z + (z + 0.5) * g.vs.z + smp.z;
-        const double u = (double)vc.mat[0] * px + (double)vc.mat[4] * py + (double)vc.mat[8] * pz + vc.mat[12];
-        umin = std::min(umin, u);
-        umax = std::max(umax, u);
-    }
-    if (!(umin > -16000.0 && umax < 16000.0)) return false;  // |256 u| < 2^22 for the tap split
+    double umin, umax;
+    if (!tap_window_holds(g, vc, smp, umin, umax)) return false;
     p.x0lo = (int)std::floor(umin - 0.5) - 2;
     p.ntaps = (int)std::floor(umax - 0.5) + 2 - p.x0lo + 1;
     p.groups = g.rx <= 4 * kBpColThreads ? 1 : 2;
@@ -580,14 +593,8 @@ bool plan_bp_block(const etcu_volume* vol, const SlabConst& g, const ViewConst* 
         const ViewConst& c = hvc[vid];
         if (!row_constant(c)) return false;
         for (int k = 0; k < nsamples; ++k) {
-            const float4& s = hsmp[(size_t)vid * nsamples + k];
-            for (int q = 0; q < 8; ++q) {
-                const double x = (q & 1) ? g.rx - 1 : 0, y = (q & 2) ? g.ry - 1 : 0, z = (q & 4) ? g.rz - 1 : 0;
-                const double u = (double)c.mat[0] * ((double)g.bmin.x + (x + 0.5) * g.vs.x + s.x) +
-                                 (double)c.mat[4] * ((double)g.bmin.y + (y + 0.5) * g.vs.y + s.y) +
-                                 (double)c.mat[8] * ((double)g.bmin.z + (z + 0.5) * g.vs.z + s.z) + c.mat[12];
-                if (!(u > -16000.0 && u < 16000.0)) return false;  // |256 u| < 2^22 for the tap split
-            }
+            double umin, umax;
+            if (!tap_window_holds(g, c, hsmp[(size_t)vid * nsamples + k], umin, umax)) return false;
         }
         span = std::max(span, std::fabs((double)c.mat[0] * g.vs.x) * (std::min(p.threads, g.rx) - 1) +
                                   std::fabs((double)c.mat[8] * g.vs.z) * (std::min(p.zper, g.rz) - 1));

@@ -102,3 +102,40 @@ def test_staged_block_matches_general_and_oracle(ctxs, shape, nviews, vpitch, wi
     require_records(*names)
     assert all("bp_parallel_kernel" in n for n in names[0])
     assert all("bp_block_kernel" in n for n in names[1])
+
+
+@pytest.mark.parametrize("samples", [1, 4])
+def test_boxes_far_along_the_rays_keep_the_general_kernels(ctxs, samples):
+    """A box four million pixels from the origin along the view's rays: its columns are the detector's, but the two
+    terms of u that cancel there are a quarter of a pixel apart in FP32, and a window bounded in
+    advance need not hold every tap.  Neither the column kernel (one sample) nor the staged one (several)
+    takes it, and the results are the general kernels'."""
+    import torch
+    from ettention_b200.operators import BackProjectionOperator, GPUMappedVolume, mrc_base_geometry
+    X, Y, Z, far = 64, 8, 16, 3.0e6
+    g = mrc_base_geometry(X, Y).rotated(45.0)
+    m = g.projection_matrix()
+    cz = float(np.round(-far * float(m[0]) / float(m[8])))
+    assert abs(float(m[0]) * far + float(m[8]) * cz) < 4.0  # u of the centre: that of a box at the origin
+    rng = np.random.Generator(np.random.PCG64(5))
+    res = torch.tensor(rng.normal(size=(Y, X)).astype(np.float32), device="cuda")
+    length = torch.tensor(rng.uniform(0.5, 30.0, size=(Y, X)).astype(np.float32), device="cuda")
+    init = rng.uniform(0.0, 1.0, size=(Z, Y, X)).astype(np.float32)
+    outs, names = [], []
+    for ctx in ctxs:
+        vol = GPUMappedVolume(ctx, (X, Y, Z), [far - 32.0, -4.0, cz - 8.0], [far + 32.0, 4.0, cz + 8.0])
+        bp = BackProjectionOperator(vol, 0.3, samples)
+        bp.setScannerGeometry(g)
+        bp.setInput(res, length, 1)
+
+        def run():
+            vol.upload(init)
+            bp.execute()
+        names.append(launched_back_projectors(run, 1))
+        outs.append(vol.download())
+        vol.close()
+    assert np.abs(outs[0] - init).max() > 0
+    assert np.array_equal(outs[1], outs[0])
+    require_records(*names)
+    assert names[0] == names[1]
+
