@@ -104,6 +104,46 @@ def test_staged_block_matches_general_and_oracle(ctxs, shape, nviews, vpitch, wi
     assert all("bp_block_kernel" in n for n in names[1])
 
 
+@pytest.mark.parametrize("order", ["identity", "maxangle"])
+def test_views_over_several_launches(ctxs, order):
+    """90 views of 9 samples: their constants exceed a launch's 32 KB (56 views), so a second one goes on with
+    the views that remain, on the volume that the first one left."""
+    from oracle import oracle as O
+    from ettention_b200 import _abi
+    from ettention_b200.operators import (AlgebraicParameterSet, BlockIterativeReconstructionOperator,
+                                          GPUMappedVolume, mrc_base_geometry)
+    from tests.helpers import oracle_geometry
+    X, Y, Z, N = 65, 4, 9, 90
+    geoms = [mrc_base_geometry(X, Y).rotated(float(a)) for a in np.linspace(-63.0, 58.0, N)]
+    rng = np.random.Generator(np.random.PCG64(N))
+    projs = rng.uniform(0.0, 4.0, size=(N, Y, X)).astype(np.float32)
+    init = rng.uniform(0.0, 1.0, size=(Z, Y, X)).astype(np.float32)
+    p = AlgebraicParameterSet(algorithm="sirt", block_size=_abi.BLOCK_ALL, iterations=1, lam=0.3, bp_samples=9,
+                              order={"identity": _abi.ORDER_IDENTITY, "maxangle": _abi.ORDER_MAXANGLE}[order])
+    outs, names = [], []
+    for ctx, launches in zip(ctxs, (1, 2)):
+        vol = GPUMappedVolume(ctx, (X, Y, Z))
+        rec = BlockIterativeReconstructionOperator(vol, geoms, projs, p, use_graph=False)
+        assert (rec.view_order() == list(range(N))) == (order == "identity")
+
+        def run():
+            vol.upload(init)
+            rec.runNiterations(1)
+        names.append(launched_back_projectors(run, launches))
+        outs.append(rec.getReconstructedVolume())
+        rec.close()
+        vol.close()
+    assert O.rel_l2(outs[1] - init, outs[0] - init) <= SAME_TOL
+    if order == "identity":
+        setup = O.ReconstructionSetup(O.VolumeGeometry.centered((X, Y, Z)), [oracle_geometry(g) for g in geoms], projs,
+                                      0.3, N, 1, 9)
+        vo = init.copy()
+        O.block_iterative(setup, vo, 1, 32)
+        assert O.rel_l2(outs[1] - init, vo - init) <= BP_TOL
+    require_records(*names)
+    assert all("bp_parallel_kernel" in n for n in names[0]) and all("bp_block_kernel" in n for n in names[1])
+
+
 @pytest.mark.parametrize("samples", [1, 4])
 def test_boxes_far_along_the_rays_keep_the_general_kernels(ctxs, samples):
     """A box four million pixels from the origin along the view's rays: its columns are the detector's, but the two
