@@ -99,7 +99,6 @@ struct etcu_recon {
     uint32_t launches = 0;
     bool persp = false;
     std::vector<int> fp_paths;      // per slab
-    std::vector<uint8_t> row_const; // per view id
     std::vector<ViewConst> hvc;     // host copy of the view constants, [slab][view id]
     std::vector<float4> hsamples;   // host copy of the sample patterns, [view id][sample]
     // fused SART step (sart_fused_kernel): per view id its tap window, per (view id,
@@ -243,12 +242,11 @@ ViewConst make_view_const(const etcu_view& v, const SlabConst& slab, float loc_l
         return a * sg;
     };
     float sdx = sdf(slab.vs.x, inv[0], r.x), sdy = sdf(slab.vs.y, inv[1], r.y), sdz = sdf(slab.vs.z, inv[2], r.z);
-    // The xz walk decodes (iz, ix) from its 32-bit offset iz * rx * ry + ix: a step off
-    // the x range must not alias a voxel of another z row (ry >= 2), and one below
-    // z = 0 must wrap past the last row ((rz + 1) * rx * ry <= 2^32).
-    const bool decodable = slab.ry >= 2 && (unsigned long long)slab.rx * (unsigned long long)slab.ry *
+    // The xz walk's offsets iz * rx * ry + ix are 32-bit; a volume of one row keeps the 3-D walk (the
+    // results are the same).
+    const bool offsets32 = slab.ry >= 2 && (unsigned long long)slab.rx * (unsigned long long)slab.ry *
                                                    (unsigned long long)(slab.rz + 1) <= (1ull << 32);
-    c.fast2d = (!v.perspective && r.y == 0.f && decodable && std::isfinite(sdx) && std::isfinite(sdy) &&
+    c.fast2d = (!v.perspective && r.y == 0.f && offsets32 && std::isfinite(sdx) && std::isfinite(sdy) &&
                 std::isfinite(sdz)) ? 1 : 0;
     return c;
 }
@@ -565,7 +563,8 @@ struct BpBlockPlan {
 //  - threads: rows of 64, 128 or 256 voxels, the width that leaves the fewest idle lanes, counting
 //    the 40 or so window entries that a block stages beside its own width;
 //  - zper: all kZ register slices, or as few as 8 while the grid would not give every
-//    multiprocessor 768 threads (its residency): a 128 x 128 x 64 block step is latency-bound.
+//    multiprocessor 768 threads (the residency of the one-sample form; 640 with several samples, 512 in
+//    blocks of 256): a 128 x 128 x 64 block step is latency-bound.
 bool plan_bp_block(const etcu_volume* vol, const SlabConst& g, const ViewConst* hvc, const float4* hsmp, int nsamples,
                    const uint32_t* vids, int n, BpBlockPlan& p) {
     etcu_context* ctx = vol->ctx;
@@ -2000,8 +1999,6 @@ etcu_status recon_build(etcu_volume* vol, const etcu_view* views, uint32_t n_vie
         }
     r->hvc = vc;
     r->hviews.assign(views, views + n_views);
-    r->row_const.resize(n_views);
-    for (uint32_t i = 0; i < n_views; ++i) r->row_const[i] = row_constant(vc[i]) ? 1 : 0;
     r->fp_paths.resize(S);
     for (size_t sl = 0; sl < S; ++sl) {
         bool all = true;

@@ -43,7 +43,7 @@ struct ViewConst {
     float mat[16];    // column-major projection matrix
     float loc_length; // long-object constant length
     int perspective;
-    int fast2d;       // parallel view with ray.y == 0, finite step differences, a decodable sub-volume
+    int fast2d;       // parallel view with ray.y == 0, finite step differences, 32-bit offsets
     int pad;
 };
 
@@ -188,8 +188,8 @@ __device__ __forceinline__ void dda_walk3(const DdaStart& st, const SlabConst& g
 // bounds every step, the walk counts its x steps and takes, while both axes have
 // that many steps left, kUnroll and then 4 steps at a time without exit tests,
 // issuing their voxel loads before their accumulations (which stay in walk order);
-// the last few steps are taken four at a time with a test each.  The 32-bit offsets
-// need ry >= 2 and (rz + 1) * rx * ry <= 2^32 (ViewConst::fast2d).
+// the last few steps are taken four at a time with a test each.  The offsets are 32-bit:
+// (rz + 1) * rx * ry <= 2^32 (ViewConst::fast2d).
 // (Recovering the budgets by decoding the voxel from the offset took nine rounds per
 // ray, each with two divisions and up to 15 single steps that waited for their loads: one
 // 96 x 96 x 96 view 13.4 us, 8.3 us in this form; 2 x 2 sub-rays over 250 x 231 x 90 in blocks
