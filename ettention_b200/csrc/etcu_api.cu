@@ -300,6 +300,7 @@ void launch_fp_m(const FpArgs& a, int path, uint32_t nviews, cudaStream_t st) {
     case kFpPathXz: launch_fp_t<VoxT, kMask, kFpPathXz>(a, nviews, st); break;
     case kFpPathXzNoCap: launch_fp_t<VoxT, kMask, kFpPathXzNoCap>(a, nviews, st); break;
     case kFpPathPerspective: launch_fp_t<VoxT, kMask, kFpPathPerspective>(a, nviews, st); break;
+    case kFpPathXzCounted: launch_fp_t<VoxT, kMask, kMask ? kFpPathXzNoCap : kFpPathXzCounted>(a, nviews, st); break;
     default: launch_fp_t<VoxT, kMask, kFpPathGeneral>(a, nviews, st); break;
     }
 }
@@ -310,11 +311,15 @@ void launch_fp_v(const FpArgs& a, bool mask, int path, uint32_t nviews, cudaStre
     else launch_fp_m<VoxT, false>(a, path, nviews, st);
 }
 
-// Walk specialisation shared by every view of a launch.
+// Walk specialisation shared by every view of a launch.  Counted steps where the lanes of a warp cannot be spread over
+// many rows: a depth of at most 100 (256 x 256 x 64, 512 x 200 x 75, 160 x 120 x 100: 0 .. 30 % less time than in rounds
+// from -60 to 45 degrees, 10 % more once, at 70) or an eighth of the width (1024 x 1024 x 128: 0 .. 7 % less); in deeper
+// volumes steep views take 20 .. 40 % more (256 x 256 x 128, 512 x 512 x 256).
 int fp_path(bool persp, bool all_fast2d, const SlabConst& slab) {
     if (persp) return kFpPathPerspective;
     if (!all_fast2d) return kFpPathGeneral;
-    return (slab.rx + slab.rz - 1 <= kMaxDdaIterations) ? kFpPathXzNoCap : kFpPathXz;
+    if (slab.rx + slab.rz - 1 > kMaxDdaIterations) return kFpPathXz;
+    return slab.rz <= 100 || 8ll * slab.rz <= slab.rx ? kFpPathXzCounted : kFpPathXzNoCap;
 }
 
 void launch_fp(const etcu_volume* vol, const FpArgs& a, int path, uint32_t nviews, cudaStream_t st) {

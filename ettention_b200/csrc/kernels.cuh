@@ -73,6 +73,10 @@ template <> __device__ __forceinline__ float load_voxel<__nv_bfloat16>(const __n
     return __bfloat162float(__ldg(p));
 }
 
+__device__ __forceinline__ float voxel_value(float v) { return v; }
+__device__ __forceinline__ float voxel_value(__half v) { return __half2float(v); }
+__device__ __forceinline__ float voxel_value(__nv_bfloat16 v) { return __bfloat162float(v); }
+
 template <typename T> __device__ __forceinline__ T store_cast(float v);
 template <> __device__ __forceinline__ float store_cast<float>(float v) { return v; }
 template <> __device__ __forceinline__ __half store_cast<__half>(float v) { return __float2half_rn(v); }
@@ -142,6 +146,12 @@ __device__ __forceinline__ bool dda_setup(float3 src, float3 ray, float3 inv, co
     return true;
 }
 
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // General 3-D Amanatides-Woo walk (DDARaytracer.hl:84-108).  kLiteral keeps the
 // reference's arithmetic step update step*sd + (1-step)*(res-dt) so that
 // non-finite step differences propagate as in the reference; otherwise the
@@ -185,17 +195,19 @@ __device__ __forceinline__ void dda_walk3(const DdaStart& st, const SlabConst& g
 //
 // The loop is restructured for memory-level parallelism without changing
 // the arithmetic: instead of re-testing the voxel index against the slab
-// bounds every step, the walk counts its x steps and takes, while both axes have
-// that many steps left, kUnroll and then 4 steps at a time without exit tests,
-// issuing their voxel loads before their accumulations (which stay in walk order);
-// the last few steps are taken four at a time with a test each.  The offsets are 32-bit:
-// (rz + 1) * rx * ry <= 2^32 (ViewConst::fast2d).
-// (Recovering the budgets by decoding the voxel from the offset took nine rounds per
-// ray, each with two divisions and up to 15 single steps that waited for their loads: one
-// 96 x 96 x 96 view 13.4 us, 8.3 us in this form; 2 x 2 sub-rays over 250 x 231 x 90 in blocks
-// of ten 5.45 -> 4.27 ms.  Large volumes are bound by L1 wavefronts, about four per warp load:
-// lanes that enter through the side face walk different z rows.)
-template <typename VoxT, bool kMask, bool kCapped = true, int kUnroll = 16>
+// bounds every step, the walk takes rounds of as many steps as neither axis can run out of,
+// kUnroll and then 4 at a time, issuing their voxel loads before their accumulations
+// (which stay in walk order); the last few steps are taken four at a time with a test each.
+// The offsets are 32-bit: (rz + 1) * rx * ry <= 2^32 (ViewConst::fast2d).
+// Large volumes are bound by L1 wavefronts, about four per warp load: lanes that enter through the side
+// face walk different z rows. The rounds bring such lanes together: each takes a share of what it has
+// left, so all of them near the exit face together and load from the same rows again (70 degrees,
+// 512 x 512 x 256: 15 sectors per load; 21 with lanes in step, dda_walk_xz_counted).  Twelve loads in
+// flight for 16-bit voxels (with sixteen 1.04 .. 1.1 times the time, a conversion between each).
+// Against the walk that recovered its budgets by two divisions a round and took a round's remainder step by
+// step, one view, tilts of -60 .. 70 degrees: 96 x 96 x 96 1.0 .. 1.4 times as fast, 512 x 512 x 256 0.97 .. 1.12
+// in FP32 and 1.03 .. 1.12 with 16-bit voxels; 61 views of 1024 x 1024 x 256 17.5 -> 15.1 ms (15.7 with lanes in step).
+template <typename VoxT, bool kMask, bool kCapped = true, int kUnroll = sizeof(VoxT) == 2 ? 12 : 16>
 __device__ __forceinline__ void dda_walk_xz(const DdaStart& st, const SlabConst& g, const VoxT* __restrict__ vol,
                                            const uint8_t* __restrict__ mask, float& acc, float& accl) {
     const unsigned plane = (unsigned)g.rx * (unsigned)g.ry;
@@ -205,15 +217,104 @@ __device__ __forceinline__ void dda_walk_xz(const DdaStart& st, const SlabConst&
     const unsigned dx = (unsigned)st.sx, dz = (unsigned)st.sz * plane;  // two's-complement deltas
     unsigned off = (unsigned)st.iz * plane + (unsigned)st.ix;  // iz * plane + ix (row carries iy)
     float rx = st.res.x, rz = st.res.z;
+    // Steps that each axis may still take before the ray leaves the slab (and the loop cap): none can
+    // run out within the next min of them.
+    int nx = st.sx > 0 ? g.rx - st.ix : (st.sx < 0 ? st.ix + 1 : 0x3fffffff);
+    int nz = st.sz > 0 ? g.rz - st.iz : (st.sz < 0 ? st.iz + 1 : 0x3fffffff);
+    int left = kMaxDdaIterations;
+    auto budget = [&]() { return kCapped ? min(min(nx, nz), left) : min(nx, nz); };
+    // One DDA step (DDARaytracer.hl:89-105): returns the segment length and the voxel it crossed.
+    auto step = [&](float& dt, unsigned& at) {
+        dt = fminf(rx, rz);
+        const bool bx = rx <= rz;
+        at = off;
+        rx = bx ? sdx : fsub(rx, dt);
+        rz = bx ? fsub(rz, dt) : sdz;
+        off += bx ? dx : dz;
+    };
+    auto add = [&](float dt, VoxT val, float mw) {
+        acc = fmaf(dt, voxel_value(val), acc);
+        if (kMask) accl = fmaf(dt, mw, accl);
+        else accl += dt;
+    };
+    // `count` unchecked steps: all voxel loads are issued before the sums, in walk order
+    auto run = [&](auto count) {
+        constexpr int kCount = decltype(count)::value;
+        float dts[kCount], mws[kCount];
+        VoxT vals[kCount];
+#pragma unroll
+        for (int j = 0; j < kCount; ++j) {
+            unsigned at;
+            step(dts[j], at);
+            vals[j] = __ldg(row + at);
+            mws[j] = kMask ? mask_weight(mrow + at) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < kCount; ++j) add(dts[j], vals[j], mws[j]);
+    };
+    // Rounds of as many steps as cannot leave the slab, 16 and 4 at a time.  Of a round's c steps, the z steps
+    // follow from the offset: off - base = (c - z) dx + z dz, the quotient far from a rounding (c <= 2^13).
+    for (int m = budget(); m >= 8; m = budget()) {
+        const unsigned base = off;
+        const int c = m & ~3;
+        for (; m >= kUnroll; m -= kUnroll) run(std::integral_constant<int, kUnroll>());
+        for (; m >= 4; m -= 4) run(std::integral_constant<int, 4>());
+        const unsigned d = off - base - (unsigned)c * dx;  // z (dz - dx), of dz's sign
+        const float per_z = (st.sz != 0 ? (float)plane : 0.f) - (float)(st.sz < 0 ? -st.sx : st.sx);
+        const int z = __float2int_rn((float)(st.sz < 0 ? 0u - d : d) * rcp_approx(per_z));
+        nx -= c - z;
+        nz -= z;
+        if (kCapped) left -= c;
+    }
+    // the last steps, four at a time with each step's own exit test
+    while (budget() > 0) {
+        float dts[4], mws[4];
+        VoxT vals[4];
+        bool live[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            live[j] = (j == 0 || live[j - 1]) && budget() > 0;
+            const bool bx = rx <= rz;
+            unsigned at;
+            step(dts[j], at);
+            vals[j] = VoxT(0.f);
+            mws[j] = 0.f;
+            if (live[j]) {
+                vals[j] = __ldg(row + at);
+                if (kMask) mws[j] = mask_weight(mrow + at);
+                nx -= bx ? 1 : 0;
+                nz -= bx ? 0 : 1;
+                if (kCapped) --left;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (live[j]) add(dts[j], vals[j], mws[j]);
+        if (!live[3]) break;
+    }
+}
+
+// The same steps and sums, for shallow volumes without mask whose rays cannot reach the loop cap: the lanes
+// of a warp go on in step while each has kUnroll steps left, counting their x steps, so a ray
+// has few short groups that wait for their loads.  Faster where the launch waits for single rays rather than
+// for L1 (one 96 x 96 x 96 view 8.3 us, 10.3 in rounds; 2 x 2 sub-rays over slabs of 250 x 231 x 23 in blocks
+// of ten 4.12 ms, 4.51 in rounds), slower where many lanes enter a deep volume through its side face (512 x 512 x
+// 256 at 70 degrees 1.4 times the time).
+template <typename VoxT, int kUnroll = 16>
+__device__ __forceinline__ void dda_walk_xz_counted(const DdaStart& st, const SlabConst& g, const VoxT* __restrict__ vol,
+                                                   float& acc, float& accl) {
+    const unsigned plane = (unsigned)g.rx * (unsigned)g.ry;
+    const VoxT* row = vol + (size_t)st.iy * (size_t)g.rx;
+    const float sdx = st.sd.x, sdz = st.sd.z;
+    const unsigned dx = (unsigned)st.sx, dz = (unsigned)st.sz * plane;  // two's-complement deltas
+    unsigned off = (unsigned)st.iz * plane + (unsigned)st.ix;  // iz * plane + ix (row carries iy)
+    float rx = st.res.x, rz = st.res.z;
     // Steps each axis may take before the ray leaves the slab, and the x steps taken so far:
-    // neither axis (nor the loop cap) can run out within the next min of what is left.
+    // neither axis can run out within the next min of what is left.
     const int nx = st.sx > 0 ? g.rx - st.ix : (st.sx < 0 ? st.ix + 1 : 0x3fffffff);
     const int nz = st.sz > 0 ? g.rz - st.iz : (st.sz < 0 ? st.iz + 1 : 0x3fffffff);
     int n = 0, nxs = 0;
-    auto budget = [&]() {
-        const int m = min(nx - nxs, nz - (n - nxs));
-        return kCapped ? min(m, kMaxDdaIterations - n) : m;
-    };
+    auto budget = [&]() { return min(nx - nxs, nz - (n - nxs)); };
     // One DDA step (DDARaytracer.hl:89-105): returns the segment length and the voxel it crossed.
     auto step = [&](float& dt, unsigned& at) {
         dt = fminf(rx, rz);
@@ -224,47 +325,44 @@ __device__ __forceinline__ void dda_walk_xz(const DdaStart& st, const SlabConst&
         off += bx ? dx : dz;
         nxs += bx ? 1 : 0;
     };
-    auto add = [&](float dt, float val, float mw) {
+    auto add = [&](float dt, float val) {
         acc = fmaf(dt, val, acc);
-        if (kMask) accl = fmaf(dt, mw, accl);
-        else accl += dt;
+        accl += dt;
     };
     // `count` unchecked steps: all voxel loads are issued before the sums, in walk order
     auto run = [&](auto count) {
         constexpr int kCount = decltype(count)::value;
-        float dts[kCount], vals[kCount], mws[kCount];
+        float dts[kCount], vals[kCount];
 #pragma unroll
         for (int j = 0; j < kCount; ++j) {
             unsigned at;
             step(dts[j], at);
             vals[j] = load_voxel(row + at);
-            mws[j] = kMask ? mask_weight(mrow + at) : 0.f;
         }
         n += kCount;
 #pragma unroll
-        for (int j = 0; j < kCount; ++j) add(dts[j], vals[j], mws[j]);
+        for (int j = 0; j < kCount; ++j) add(dts[j], vals[j]);
     };
     while (budget() >= kUnroll) run(std::integral_constant<int, kUnroll>());
     while (budget() >= 4) run(std::integral_constant<int, 4>());
     // the last steps, four at a time with each step's own exit test
     while (budget() > 0) {
-        float dts[4], vals[4], mws[4];
+        float dts[4], vals[4];
         bool live[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             live[j] = (j == 0 || live[j - 1]) && budget() > 0;
             unsigned at;
             step(dts[j], at);
-            vals[j] = mws[j] = 0.f;
+            vals[j] = 0.f;
             if (live[j]) {
                 vals[j] = load_voxel(row + at);
-                if (kMask) mws[j] = mask_weight(mrow + at);
                 ++n;
             }
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (live[j]) add(dts[j], vals[j], mws[j]);
+            if (live[j]) add(dts[j], vals[j]);
         if (!live[3]) break;
     }
 }
@@ -414,8 +512,10 @@ struct FpArgs {
 
 // kPath: kFpPathGeneral parallel rays (walk chosen per ray), kFpPathXz / kFpPathXzNoCap
 // parallel views tilted about y (xz walk; the loop cap is dropped when the sub-volume
-// cannot reach it, rx + rz - 1 <= 2048 steps), kFpPathPerspective.
-enum FpPath : int { kFpPathGeneral = 0, kFpPathXz = 1, kFpPathXzNoCap = 2, kFpPathPerspective = 3 };
+// cannot reach it, rx + rz - 1 <= 2048 steps; kFpPathXzCounted: the counted walk), kFpPathPerspective.
+enum FpPath : int {
+    kFpPathGeneral = 0, kFpPathXz = 1, kFpPathXzNoCap = 2, kFpPathPerspective = 3, kFpPathXzCounted = 4
+};
 
 // Projection epilogue of one detector pixel (ForwardProjectionKernel /
 // VirtualProjection.cl:8-9 / Compare.cl:8): normalise by the sub-ray count and
@@ -492,7 +592,8 @@ __device__ __forceinline__ void fp_pixel(const FpArgs& a, uint32_t first, int p,
                     } else {
                         DdaStart st;
                         if (dda_setup(s, ray, inv, a.slab, st))
-                            dda_walk_xz<VoxT, kMask, kPath == kFpPathXz>(st, a.slab, vol, a.mask, v, l);
+                            if constexpr (kPath == kFpPathXzCounted) dda_walk_xz_counted<VoxT>(st, a.slab, vol, v, l);
+                            else dda_walk_xz<VoxT, kMask, kPath == kFpPathXz>(st, a.slab, vol, a.mask, v, l);
                     }
                     accv += v;
                     accl += l;
@@ -531,7 +632,7 @@ __device__ __forceinline__ void fp_pixel(const FpArgs& a, uint32_t first, int p,
 // latency-bound: 8 x 4 warps per SM cut the C3 forward projection by 19 % against 4),
 // 4 otherwise.
 template <typename VoxT, bool kMask, int kPath>
-__global__ void __launch_bounds__(128, (kPath == kFpPathXz || kPath == kFpPathXzNoCap) ? 7
+__global__ void __launch_bounds__(128, (kPath == kFpPathXz || kPath == kFpPathXzNoCap || kPath == kFpPathXzCounted) ? 7
                                            : (kPath == kFpPathPerspective ? 8 : 4))
     forward_project_kernel(const __grid_constant__ FpArgs a) {
     const int v = a.beside ? (int)blockIdx.y : (int)blockIdx.z, row = a.beside ? (int)blockIdx.z : (int)blockIdx.y;
@@ -597,12 +698,6 @@ struct BpView {
 
 __host__ __device__ constexpr size_t bp_smem_bytes(int nviews, int nsamples) {
     return ((size_t)nviews * sizeof(BpView) + 15) / 16 * 16 + (size_t)nviews * (size_t)nsamples * sizeof(float4);
-}
-
-__device__ __forceinline__ float rcp_approx(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
 }
 
 // a / b to within one ulp: reciprocal estimate, one Newton correction of the quotient.

@@ -10,6 +10,7 @@ edges of their tiles and of the rules that select them.
 * bp_block_kernel for one view (rows that the column kernel does not take, from the size
   at which they fill the chip) against bp_sart_row_kernel: the detector rows are blended first, a few
   ulps per update: SAME_TOL.  Each one's own error is held to a 64-bit restatement.
+* the forward projector's counted walk (shallow volumes) against its walk in rounds.
 * several views of one launch side by side against each view in a launch of its own.
 * the persistent fused SART step's narrow rows (several groups of threads on a chunk's
   slices) against the unfused kernels: bit-identical, widths around whole warps and the half
@@ -296,6 +297,40 @@ def test_narrow_fused_rows_are_bit_identical_to_unfused(shape, storage):
     assert np.abs(outs[0][0] - init).max() > 0
     assert np.array_equal(outs[1][0], outs[0][0])
     assert outs[1][1] == pytest.approx(outs[0][1], rel=1e-12)
+
+
+@pytest.mark.parametrize("shape", [(4, 5, 3), (64, 6, 100), (70, 5, 33), (130, 3, 97), (900, 2, 112), (37, 4, 101),
+                                   (64, 3, 260)])
+@pytest.mark.parametrize("storage", ["float32", "bf16_master", "half"])
+def test_forward_walks_are_bit_identical(ctxs, shape, storage):
+    """Volumes up to 100 slices deep, or an eighth of their width, take the counted walk; a mask of ones
+    sends them to the walk in rounds with the same weights.  The last two shapes take the rounds both ways,
+    with and without mask (depths around the line)."""
+    import torch
+    from ettention_b200 import _abi
+    from ettention_b200.operators import ForwardProjectionOperator, GPUMappedVolume, mrc_base_geometry
+    X, Y, Z = shape
+    kind = {"float32": _abi.VOXEL_FLOAT32, "bf16_master": _abi.VOXEL_BF16_MASTER, "half": _abi.VOXEL_HALF16}[storage]
+    rng = np.random.Generator(np.random.PCG64(X + Z))
+    init = rng.uniform(0.0, 1.0, size=(Z, Y, X)).astype(np.float32)
+    for samples in (1, 2):
+        images = []
+        for mask in (None, np.full((Z, Y, X), 255, np.uint8)):
+            vol = GPUMappedVolume(ctxs[1], shape, voxel_type=kind)
+            vol.upload(init)
+            if mask is not None:
+                vol.set_mask(mask)
+            op = ForwardProjectionOperator(vol, samples)
+            for tilt in (-89.5, -61.0, -30.3, 0.0, 12.5, 45.0, 70.0, 90.0, 135.0, 180.0, 233.0):
+                v, length = (torch.zeros((Y, X), device="cuda") for _ in range(2))
+                op.setScannerGeometry(mrc_base_geometry(X, Y).rotated(tilt))
+                op.SetOutput(v, length)
+                op.Execute(0)
+                images.append(torch.stack([v, length]).cpu().numpy())
+            vol.close()
+        n = len(images) // 2
+        assert all(i.max() > 0 for i in images)
+        assert all(np.array_equal(a, b) for a, b in zip(images[:n], images[n:]))
 
 
 @pytest.mark.parametrize("perspective", [False, True])
