@@ -914,7 +914,7 @@ def run_c3(args, steps=None, warmup=None, cpu_baseline=True):
                          "forward_project": {"kernel": "forward_project_kernel (perspective walk)",
                                              "algorithmic_bytes": fp_bytes,
                                              "frac": fp_bytes / (fp_ms * 1e-3) / 1e9 / hbm},
-                         "back_project": {"kernel": "bp_perspective_kernel", "algorithmic_bytes": bp_bytes,
+                         "back_project": {"kernel": "bp_persp_row_kernel", "algorithmic_bytes": bp_bytes,
                                           "frac": bp_bytes / (bp_ms * 1e-3) / 1e9 / hbm}}},
         "cpu_baseline": cpu, "clocks": clk.summary()}
 
@@ -1037,7 +1037,7 @@ def run_c5(args):
                    "network": "3-level 3-D conv encoder-decoder 16/32/64, BF16, FP32 accumulate",
                    "trained": {k: (v.tolist() if hasattr(v, "tolist") else v) for k, v in meta.items()
                                if k in ("series", "epochs", "lr", "train_seed0")}},
-        "roofline": {"bound": "tensor", "kernel": "conv_tc_kernel (network inference)", "flops_per_inference": flops,
+        "roofline": {"bound": "tensor", "kernel": "conv_zfold_kernel, conv_tc_kernel (network inference)", "flops_per_inference": flops,
                      "achieved": flops / (net_ms * 1e-3) / 1e12, "peak": tf_peak, "unit": "TFLOP/s",
                      "frac": flops / (net_ms * 1e-3) / 1e12 / tf_peak, "net_ms": net_ms},
         "clocks": clk.summary(), "per_seed": per[:8]}

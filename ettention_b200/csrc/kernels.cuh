@@ -2639,8 +2639,8 @@ __global__ void __launch_bounds__(32 * kBpRowWarps, kBpRowBlocks) bp_persp_row_k
 // convolution directly, one output row of one view per block: the padded source row and the taps
 // are staged in shared memory, Wu is a power of two (a mask wraps the position), and a thread
 // sums four pixels a block width apart, so a tap is loaded once for four multiply-adds.  All views
-// go in one launch (61 views of 512 x 512: 2.2 ms less of a WBP call of 8.1 ms than with a launch per view, two
-// remainders and three loads per tap).  It also writes the
+// go in one launch (61 views of 512 x 512: 1.86 ms with a launch per view, two remainders and three loads
+// per tap, 0.24 ms in this form).  It also writes the
 // pixel's ray length through the complete volume (ComputeRayLength.cl) beside the
 // filtered value, the (residual, length) pair the back projector reads.
 struct WbpArgs {

@@ -869,8 +869,9 @@ __global__ void relayout_zfold_backward_kernel(const float* __restrict__ W, int 
 // step and one thread issued 216 MMAs per tile: 3.6 ms for a 16 -> 16 layer at 256 x 256 x
 // 128.  This form took 0.76 ms with 16-byte cells as the copies' inner dimension (one cell per
 // clock) and 0.24 ms with rows of 2 KB (tma_load_4d of a 64-bit view of the tensor; moving by
-// a cell is two elements, 16 bytes).  What bounds it is the operands' way from L2: 48 KB per
-// tile of 128 voxels (3.1 GB, 13 TB/s), against 0.54 GB (0.08 ms) from DRAM.
+// a cell is two elements, 16 bytes).  What bounds it is the operands' way from L2 (48 KB per
+// tile of 128 voxels, 2.7 GB by the L2's count, 10.8 TB/s) and the tensor pipe (60 % active), against 0.54 GB
+// (0.08 ms) from DRAM.
 struct WgradArgs {
     int X, Y, Z, batch;
     int in_c8;             // chunks per batch item of the input tensor
