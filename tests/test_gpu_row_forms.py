@@ -13,8 +13,8 @@ edges of their tiles and of the rules that select them.
 * the forward projector's counted walk (shallow volumes) against its walk in rounds.
 * several views of one launch side by side against each view in a launch of its own.
 * the persistent fused SART step's narrow rows (several groups of threads on a chunk's
-  slices) against the unfused kernels: bit-identical, widths around whole warps and the half
-  block at which the wide form takes over.
+  slices) against the unfused kernels: bit-identical, widths around whole warps and the 256 voxels
+  from which the wide form takes over.
 * input gradients on the z-streamed convolution against the per-tap kernel (ETCU_CONV_ZFOLD=0):
   two orders of FP32 sums whose BF16 roundings flip here and there, within the bar that both keep to
   the oracle."""
